@@ -425,6 +425,22 @@ __device__ __forceinline__ bool warp_run_sum(long long key, T (&v)[NV]) {
   return head && key >= 0;
 }
 
+// ------------------------------------------------------------ exact division
+// a / b from y = RN(1/b), correctly rounded (Markstein, "Computation of
+// elementary functions on the IBM RISC System/6000 processor", IBM J. Res.
+// Dev. 34, 1990: with y the rounded reciprocal and q within an ulp of a / b,
+// RN(q + RN(a - b q) y) is RN(a / b)): a y is within two ulps, one correction
+// brings it within one, the second rounds it (a zero keeps its sign, a NaN
+// stays one).  The remainders are exact for 1e-280 < |a| < 1e200 with a
+// 1e-100 < |b| < 1e100; a smaller a may end one ulp off, from a larger one
+// the result is not a number.  A branch to the division for those would cost
+// the callers' loops their registers.
+__device__ __forceinline__ double div_by(double a, double b, double y) {
+  const double q0 = a * y;
+  const double q1 = __fma_rn(__fma_rn(-b, q0, a), y, q0);
+  return __fma_rn(__fma_rn(-b, q1, a), y, q1);
+}
+
 // ------------------------------------------------ async copies and mbarriers
 __device__ __forceinline__ uint32_t smem_addr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 

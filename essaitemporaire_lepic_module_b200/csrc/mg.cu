@@ -26,7 +26,7 @@
 // (Src/mg.f90:314-805); the Dirichlet instance is unchanged.
 #include <cooperative_groups.h>
 
-#include "lepic_internal.cuh"
+#include "mgsplit.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -565,6 +565,449 @@ __global__ void __launch_bounds__(MG_BLOCK) k_pdesolver(const MGArgs *__restrict
   }
 }
 
+// ------------------------------------------------ colour-split Dirichlet solve
+// The same schedule and the same node arithmetic on colour-split levels
+// (mgsplit.cuh), for Dirichlet walls.  What it changes is how many grid
+// barriers a sweep costs and what a phase reads:
+//   * a sweep is two phases, red and black, and no third one for its residual:
+//     the black nodes' share is summed in the black phase (their neighbours
+//     are final there) and the red nodes' share in the next sweep's red phase,
+//     which writes its new values into a second buffer that is dropped when
+//     the residual ends the smoothing;
+//   * a residual that nothing reads (that of the fourth sweep, but for the
+//     last smoothing of a cycle) is not computed;
+//   * the levels that fit the shared memory of one SM are smoothed there by
+//     block 0.
+// Measured (cold solves to 1e-10): 128^3 with electrodes 13.8 -> 4.4 ms (13
+// cycles; a red or black phase of level 1 takes 8 us for the 52 MB it moves
+// through L2, one of a small level 2.9 us, 1.2 of them the barrier), 40x24x32
+// 1.17 -> 0.46 ms, 96^3 warm 4.5 -> 1.0 ms.  What bounds it: L2 traffic on the
+// finest level, barriers and the latency of dependent FP64 operations below.
+// 512 threads: with 768 and 1024 the phases spill (128^3: 4.8 and 5.8 ms).
+constexpr int SP_BLOCK = 512;
+constexpr size_t SP_CHIP = 227000;   // shared memory of the levels on chip: 16^3 and below
+
+struct SPArgs {
+  mgs::Lev<double> L[MG_MAX + 2];   // levels 1..ng; after them level ls + 1 with its arrays on the grid
+  unsigned oc[MG_MAX + 1];          // levels ls+1..ng: byte offset of their arrays on chip
+  unsigned ol;                      // and of the level descriptors
+  int ng, ls, ncycl;
+  double alpha, eps, omega;
+  double *u;                  // the caller's grid arrays
+  const double *b;
+  const int *bc;
+  double *partial;            // [2][gridDim.x]
+  int *out_i;
+  double *out_d;
+};
+
+extern __shared__ __align__(16) unsigned char sp_smem[];
+
+// the descriptors, copied to shared memory by every block: read from the
+// kernel's parameters level by level they cost microseconds of constant-cache
+// misses per smoothing call
+__device__ __forceinline__ const mgs::Lev<double> &lev(const SPArgs &a, int l) {
+  return reinterpret_cast<const mgs::Lev<double> *>(sp_smem + a.ol)[l - 1];
+}
+
+// deterministic sum over the team of one value per thread in two steps: each
+// caller's share into slot `set` before a barrier, the total after it (every
+// warp adds the shares up in the same order)
+template <bool GRID>
+__device__ __forceinline__ void share(double v, int set, double *sh, double *partial) {
+  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+  v = warp_sum(v);
+  if (!GRID) {
+    if (lane == 0) sh[32 * set + wp] = v;
+    return;
+  }
+  if (lane == 0) sh[wp] = v;
+  __syncthreads();
+  if (wp == 0) {
+    v = lane < (int)(blockDim.x >> 5) ? sh[lane] : 0.0;
+    v = warp_sum(v);
+    if (lane == 0) partial[set * gridDim.x + blockIdx.x] = v;
+  }
+}
+template <bool GRID>
+__device__ __forceinline__ double total(int set, const double *sh, const double *partial) {
+  const int lane = threadIdx.x & 31;
+  double v = 0.0;
+  if (GRID) {
+    for (int q = lane; q < (int)gridDim.x; q += 32) v += partial[set * gridDim.x + q];
+  } else {
+    v = lane < (int)(blockDim.x >> 5) ? sh[32 * set + lane] : 0.0;
+  }
+  return warp_sum(v);
+}
+
+// level l on the grid / on chip (block 0)
+template <bool GRID>
+__device__ __forceinline__ const mgs::Lev<double> &level_of(const SPArgs &a, int l) {
+  return lev(a, GRID && l == a.ls + 1 ? a.ng + 1 : l);
+}
+// the red half of a level's residual: below level 1 it lies in the red buffer
+// that is not current (walls and ghosts are 0 in both)
+__device__ __forceinline__ double *residual_red(const mgs::Lev<double> &L, int cur) {
+  return L.rf[mgs::RED] ? L.rf[mgs::RED] : L.red[cur ^ 1];
+}
+
+// Src/sors.f90:1-535: up to four sweeps (the coarsest level of the first
+// cycle: until res <= eps_abs), ended early when a sweep's residual is at
+// most 0.6 of the one before; cur: the current red buffer.  The residual of
+// sweep l - 1 is known after the red phase of sweep l.  Returns the last
+// sweep's residual when need_res, the sweeps done in ksor.  started: the
+// restriction has done the first sweep's red phase.
+template <bool GRID>
+__device__ __forceinline__ double smooth(const SPArgs &a, int level, int &cur, bool first, int dig, bool need_res,
+                                         bool started, cg::grid_group &grid, double *sh, int &ksor) {
+  using namespace mgs;
+  const Lev<double> &L = level_of<GRID>(a, level);
+  const Team w = GRID ? grid_team() : block_team();
+  const double om = a.omega, eps_abs = a.alpha * a.eps;
+  const int nr = (first && dig == 0) ? 1000000 : 4;
+  auto barrier = [&]() {
+    if (GRID)
+      grid.sync();
+    else
+      __syncthreads();
+  };
+  double res = 0.0, part = 0.0;
+  bool stopped = false;
+  ksor = nr;
+  for (int l = 1; l <= nr; ++l) {
+    if (l == 1 && started) {
+      cur ^= 1;   // taken back below: the values stand in the current buffer
+    } else if (l == 1) {
+      colour_phase<double, 2, RED, DO_RELAX>(L, L.red[cur], L.red[cur ^ 1], L.black, om, w);
+      barrier();
+    } else {
+      part += colour_phase<double, 2, RED, DO_RELAX | DO_RES>(L, L.red[cur], L.red[cur ^ 1], L.black, om, w);
+      share<GRID>(part, l & 1, sh, a.partial);
+      barrier();
+      if (dig == 0) {
+        res = total<GRID>(l & 1, sh, a.partial);
+        stopped = res <= eps_abs;
+      } else if (l >= 3) {
+        const double before = l == 3 ? total<GRID>((l - 1) & 1, sh, a.partial) : res;
+        res = total<GRID>(l & 1, sh, a.partial);
+        stopped = before > 0.0 && res / before <= 0.6;
+      }
+      if (stopped) {
+        ksor = l - 1;
+        break;
+      }
+    }
+    cur ^= 1;
+    if (l < nr || need_res)
+      part = colour_phase<double, 2, BLACK, DO_RELAX | DO_RES>(L, L.black, L.black, L.red[cur], om, w);
+    else
+      colour_phase<double, 2, BLACK, DO_RELAX>(L, L.black, L.black, L.red[cur], om, w);
+    barrier();
+  }
+  if (need_res && !stopped) {
+    part += colour_phase<double, 2, RED, DO_RES>(L, L.red[cur], nullptr, L.black, om, w);
+    share<GRID>(part, 1, sh, a.partial);   // sweep 4 (l = 5)
+    barrier();
+    res = total<GRID>(1, sh, a.partial);
+  }
+  return res;
+}
+
+// the residual of a level weighted onto the next one
+template <bool GRID>
+__device__ __forceinline__ void restrict_level(const SPArgs &a, int level, int cur, bool masks, cg::grid_group &grid) {
+  using namespace mgs;
+  const Lev<double> &F = level_of<GRID>(a, level), &C = level_of<GRID>(a, level + 1);
+  double *R = residual_red(F, cur);
+  const Team w = GRID ? grid_team() : block_team();
+  residual_colour<double, 2, RED>(F, F.red[cur], F.black, R, w);
+  residual_colour<double, 2, BLACK>(F, F.black, F.red[cur], F.rf[BLACK], w);
+  if (GRID)
+    grid.sync();
+  else
+    __syncthreads();
+  restrict_to<double>(F, C, R, F.rf[BLACK], masks, true, a.omega, w);
+  if (GRID)
+    grid.sync();
+  else
+    __syncthreads();
+}
+
+// the part of a V-cycle on the levels on chip, by block 0
+__device__ __forceinline__ void chip_cycle(const SPArgs &a, bool first, int *iter, cg::grid_group &grid, double *sh) {
+  using namespace mgs;
+  const int top = a.ls + 1, ng = a.ng, t0 = threadIdx.x, bd = blockDim.x;
+  int cur[MG_MAX + 1];
+  const Lev<double> &X = level_of<true>(a, top);
+  {
+    const Lev<double> &L = level_of<false>(a, top);
+    for (int e = t0; e < L.len; e += bd) {
+      L.b[0][e] = X.b[0][e];
+      L.b[1][e] = X.b[1][e];
+      L.red[0][e] = X.red[0][e];   // the first red phase is done
+      L.black[e] = 0.0;
+      if (first || e < L.HN || e >= L.HN * (L.n3 + 2)) L.red[1][e] = 0.0;   // planes no red phase writes
+      if (first) {
+        L.m[e] = X.m[e];
+        if (L.rf[BLACK]) L.rf[BLACK][e] = 0.0;
+      }
+    }
+    __syncthreads();
+  }
+  // down to the coarsest level and up again (one call site per step: the
+  // loops keep their registers)
+  const int mid = ng - top;
+  for (int g = 0; g <= 2 * mid; ++g) {
+    const int l = g <= mid ? top + g : ng - (g - mid);
+    if (g <= mid) cur[l] = 0;
+    if (g > mid) {
+      const Lev<double> &F = level_of<false>(a, l), &C = level_of<false>(a, l + 1);
+      prolong_to<double>(F, C, F.red[cur[l]], F.red[cur[l] ^ 1], C.red[cur[l + 1]], block_team());
+      __syncthreads();
+    }
+    int k = 0;
+    smooth<false>(a, l, cur[l], first, g <= mid ? l - ng : ng - l, false, g <= mid, grid, sh, k);
+    iter[l] += k;
+    if (g < mid) restrict_level<false>(a, l, cur[l], first, grid);
+  }
+  const Lev<double> &L = level_of<false>(a, top);
+  for (int e = t0; e < L.len; e += bd) {
+    X.red[0][e] = L.red[cur[top]][e];
+    X.black[e] = L.black[e];
+  }
+}
+
+// the caller's grids into the split arrays of level 1 and back
+__device__ __noinline__ void split_in(const SPArgs &a) {
+  using namespace mgs;
+  const Lev<double> &L = lev(a, 1);
+  const long long N1 = L.n1 + 3, R1 = L.n1 + 2, R2 = L.n2 + 2;
+  const int last = L.n1 + 2;
+  elements(L, grid_team(), [&](int e, int ii, int j, int k) {
+    // the row's nodes i = 2 ii and 2 ii + 1: one of each colour
+    const long long q = 2 * ii + N1 * (j + (long long)L.N2 * k), qb = 2 * ii + R1 * (j + R2 * (long long)k);
+    const bool jk = j >= 1 && k >= 1 && j <= L.n2 + 1 && k <= L.n3 + 1;
+    const int odd = (j + k + 1) & 1;   // the colour of i odd is RED when j + k is even
+    unsigned m = 0;
+#pragma unroll
+    for (int x = 0; x < 2; ++x) {
+      const int i = 2 * ii + x, c = x ? odd ^ 1 : odd;
+      double u = 0.0, b = 0.0;
+      unsigned bits = x ? MB_ODD : 0;
+      if (i <= last) {
+        u = a.u[q + x];
+        const int bc = a.bc[q + x];
+        if (bc <= 0) bits |= MB_FREE;
+        if (jk && i >= 1 && i <= L.n1 + 1) {
+          b = a.b[qb + x];
+          bits |= (bc <= 0 ? MB_UPD : 0) | (bc == -1 ? MB_PLASMA : 0);
+        }
+      }
+      m |= MB(c, bits);
+      L.b[c][e] = b;
+      if (L.rf[c]) L.rf[c][e] = 0.0;
+      (c == RED ? L.red[0] : L.black)[e] = u;
+      if (c == RED) L.red[1][e] = u;
+    }
+    L.m[e] = (unsigned char)m;
+  });
+}
+__device__ __noinline__ void split_out(const SPArgs &a, int cur) {
+  using namespace mgs;
+  const Lev<double> &L = lev(a, 1);
+  const double *red = L.red[cur];
+  elements(L, grid_team(), [&](int e, int ii, int j, int k) {
+    const unsigned m = L.m[e];
+    const int odd = (j + k + 1) & 1;
+    double *u = a.u + 2 * ii + (long long)(L.n1 + 3) * (j + (long long)L.N2 * k);
+#pragma unroll
+    for (int x = 0; x < 2; ++x) {
+      const int c = x ? odd ^ 1 : odd;
+      if (m & MB(c, MB_FREE)) u[x] = c == RED ? red[e] : L.black[e];
+    }
+  });
+}
+
+__global__ void __launch_bounds__(SP_BLOCK, 1) k_pdesolver_split(const __grid_constant__ SPArgs a) {
+  using namespace mgs;
+  cg::grid_group grid = cg::this_grid();
+  __shared__ double sh[64];
+  const int ng = a.ng, ls = a.ls, down = ls < ng ? ls : ng - 1;   // down: the last grid level restricted from
+  unsigned curs = 0;   // bit l: the current red buffer of grid level l
+  {
+    const int words = (int)(sizeof(Lev<double>) / 4) * (ng + 1);
+    const unsigned *from = reinterpret_cast<const unsigned *>(a.L + 1);
+    for (int q = threadIdx.x; q < words; q += blockDim.x) reinterpret_cast<unsigned *>(sp_smem + a.ol)[q] = from[q];
+    __syncthreads();
+    // the levels on chip: their arrays in this block's shared memory
+    const int l = ls + 1 + threadIdx.x;
+    if (l <= ng) {
+      Lev<double> &L = const_cast<Lev<double> &>(lev(a, l));
+      double *p = reinterpret_cast<double *>(sp_smem + a.oc[l]);
+      const int n = L.len;
+      L.red[0] = p;
+      L.red[1] = p + n;
+      L.black = p + 2 * n;
+      L.b[0] = p + 3 * n;
+      L.b[1] = p + 4 * n;
+      L.rf[BLACK] = l == ng ? nullptr : p + 5 * n;
+      L.m = reinterpret_cast<unsigned char *>(p + (l == ng ? 5 : 6) * n);
+    }
+  }
+  __syncthreads();
+  split_in(a);
+  grid.sync();
+  double res_s = 0.0, ktot = 0.0, r = 0.0;
+  int status = 0, k = 1;
+  bool converged = false;
+  while (!converged) {
+    const bool first = k == 1;
+    int iter[MG_MAX + 1];
+    for (int i = 0; i <= MG_MAX; ++i) iter[i] = 0;
+    // grid levels down, the coarsest level or the levels on chip, grid levels
+    // up (one call site per step)
+    const int mid = down + 1;
+    for (int g = 1; g <= 2 * down + 1; ++g) {
+      if (g == mid && ls < ng) {
+        if (blockIdx.x == 0) chip_cycle(a, first, iter, grid, sh);
+        grid.sync();
+        continue;
+      }
+      const int l = g <= mid ? g : 2 * mid - g;
+      int cur = (curs >> l) & 1, ks = 0;
+      if (g > mid) {
+        const Lev<double> &F = level_of<true>(a, l), &C = level_of<true>(a, l + 1);
+        prolong_to<double>(F, C, F.red[cur], F.red[cur ^ 1], C.red[(curs >> (l + 1)) & 1], grid_team());
+        grid.sync();
+      }
+      r = smooth<true>(a, l, cur, first, g <= mid ? l - ng : ng - l, g == 2 * down + 1, g > 1 && g <= mid, grid, sh,
+                       ks);
+      iter[l] += ks;
+      curs = (curs & ~(1u << l)) | ((unsigned)cur << l);
+      if (g < mid) {
+        restrict_level<true>(a, l, cur, first, grid);
+        curs &= ~(2u << l);   // level l + 1 starts in its first buffer
+      }
+    }
+    for (int i = 1; i <= ng; ++i) ktot = ktot + (double)(float)iter[i] / exp2((double)(2 * (i - 1)));
+    r = r / a.alpha;
+    if (first) {
+      res_s = r;
+    } else if (fabs(r / res_s) > 10.0) {
+      status = LEPIC_ERR_DIVERGED;
+      converged = true;
+    }
+    if (r < a.eps || k == a.ncycl) converged = true;
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+      for (int i = 1; i <= ng; ++i) a.out_i[2 + i] = iter[i];
+    k = k + 1;
+  }
+  split_out(a, (curs >> 1) & 1);
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    a.out_i[0] = k;
+    a.out_i[1] = status;
+    a.out_d[0] = ktot;
+    a.out_d[1] = r;
+  }
+}
+
+// the solve's results to the host: waits for the stream, returns the status
+int solve_results(const int *out_i, const double *out_d, int *k_out, double *ktot_out, double *res_out,
+                  cudaStream_t s) {
+  int hi[2];
+  double hd[2];
+  LEPIC_CUDA(cudaMemcpyAsync(hi, out_i, sizeof(hi), cudaMemcpyDeviceToHost, s));
+  LEPIC_CUDA(cudaMemcpyAsync(hd, out_d, sizeof(hd), cudaMemcpyDeviceToHost, s));
+  LEPIC_CUDA(cudaStreamSynchronize(s));
+  if (k_out) *k_out = hi[0];
+  if (ktot_out) *ktot_out = hd[0];
+  if (res_out) *res_out = hd[1];
+  return hi[1];
+}
+
+// The split solve's arrays and launch; LEPIC_OK with launched = false where it
+// does not apply (a level with too many nodes for its 32-bit element numbers,
+// coefficients out of div_by's range): the caller takes the general kernel.
+int launch_split(const int n[3], const double h[3], double *u, const double *b, const int *bcnd, int ncycl,
+                 double eps, double omega, int ng, double eps0, int *out_i, double *out_d, cudaStream_t s,
+                 bool &launched) {
+  using Lev = mgs::Lev<double>;
+  launched = false;
+  if (Lev::elements(n[0], n[1], n[2]) >= 1200000000LL) return LEPIC_OK;
+  SPArgs A;
+  memset(&A, 0, sizeof(A));
+  A.ng = ng;
+  A.ncycl = ncycl;
+  A.eps = eps;
+  A.omega = omega;
+  A.u = u;
+  A.b = b;
+  A.bc = bcnd;
+  A.out_i = out_i;
+  A.out_d = out_d;
+  for (int l = 1; l <= ng; ++l) {
+    Lev &L = A.L[l];
+    L.shape(n[0] >> (l - 1), n[1] >> (l - 1), n[2] >> (l - 1));
+    double hl[3];
+    for (int q = 0; q < 3; ++q) hl[q] = h[q] * (double)(1 << (l - 1));
+    L.aw = eps0 / (hl[0] * hl[0]);
+    L.an = eps0 / (hl[1] * hl[1]);
+    L.at = eps0 / (hl[2] * hl[2]);
+    L.ac = -(L.an + L.an + L.aw + L.aw + L.at + L.at);
+    L.rac = 1.0 / L.ac;
+  }
+  if (!(fabs(A.L[1].ac) < 1e100 && fabs(A.L[ng].ac) > 1e-100)) return LEPIC_OK;   // div_by's range
+  // the levels that fit on chip (level 1 stays on the grid): per element two
+  // red and one black value, b of both, the black residual, one byte
+  size_t csm = 0;
+  A.ls = ng;
+  for (int l = ng; l >= 2; --l) {
+    const size_t need = ((size_t)A.L[l].len * (8 * (l == ng ? 5 : 6) + 1) + 15) & ~(size_t)15;
+    if (csm + need > SP_CHIP) break;
+    A.oc[l] = (unsigned)csm;
+    csm += need;
+    A.ls = l - 1;
+  }
+  A.ol = (unsigned)csm;
+  csm += sizeof(Lev) * (ng + 1);
+  if (A.ls < ng) A.L[ng + 1] = A.L[A.ls + 1];
+  for (int l = 1; l <= A.ls + 1 && l <= ng; ++l) {
+    Lev &L = A.L[l <= A.ls ? l : ng + 1];
+    // one allocation per level: red twice, black, b twice, and on the levels
+    // that restrict the residual (its red half in the spare red buffer but
+    // on level 1, whose walls are not 0)
+    const size_t n8 = (size_t)L.len;
+    const bool restricts = l <= A.ls && l < ng;
+    const int halves = 5 + (restricts ? (l == 1 ? 2 : 1) : 0);
+    char nm[32];
+    snprintf(nm, sizeof nm, "mgs_%d", l);
+    double *p = (double *)scratch(nm, (sizeof(double) * halves + 1) * n8);
+    if (!p) return LEPIC_ERR_CUDA;
+    L.red[0] = p;
+    L.red[1] = p + n8;
+    L.black = p + 2 * n8;
+    L.b[0] = p + 3 * n8;
+    L.b[1] = p + 4 * n8;
+    if (restricts) {
+      L.rf[mgs::BLACK] = p + 5 * n8;
+      if (l == 1) L.rf[mgs::RED] = p + 6 * n8;
+    }
+    L.m = reinterpret_cast<unsigned char *>(p + halves * n8);
+  }
+  A.alpha = fabs((double)((n[0] + 1) * (n[1] + 1) * (n[2] + 1)) * A.L[1].ac) * 1.0;
+  const int blocks = ctx().sms;
+  A.partial = (double *)scratch("mgs_partial", sizeof(double) * 2 * blocks);
+  if (!A.partial) return LEPIC_ERR_CUDA;
+  LEPIC_CUDA(cudaFuncSetAttribute(k_pdesolver_split, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csm));
+  void *args[] = {&A};
+  int tm = timer_start("pdesolver_f64", s);
+  LEPIC_CUDA(cudaLaunchCooperativeKernel((void *)k_pdesolver_split, dim3(blocks), dim3(SP_BLOCK), args, csm, s));
+  timer_stop(tm, s);
+  launched = true;
+  return LEPIC_OK;
+}
+
 }  // namespace
 
 int launch_pdesolver(const Dims &d, const double h[3], double *u, const double *b, const int *bcnd,
@@ -576,6 +1019,13 @@ int launch_pdesolver(const Dims &d, const double h[3], double *u, const double *
   for (int a = 0; a < 3; ++a)
     if (n[a] % (1 << (ng - 1))) return LEPIC_ERR_ARG;
   Ctx &c = ctx();
+  int *out_i = (int *)scratch("mg_out_i", sizeof(int) * (MG_MAX + 4));
+  double *out_d = (double *)scratch("mg_out_d", sizeof(double) * 2);
+  if (!out_i || !out_d) return LEPIC_ERR_CUDA;
+  bool launched = false;
+  if (!gen)
+    if (int rc = launch_split(n, h, u, b, bcnd, ncycl, eps, omega, ng, eps0, out_i, out_d, s, launched)) return rc;
+  if (launched) return solve_results(out_i, out_d, k_out, ktot_out, res_out, s);
   MGArgs A;
   memset(&A, 0, sizeof(A));
   A.ng = ng;
@@ -639,9 +1089,9 @@ int launch_pdesolver(const Dims &d, const double h[3], double *u, const double *
   int blocks = c.sms * (occ < 2 ? occ : 2);
   A.partial = (double *)scratch("mg_partial", sizeof(double) * blocks);
   A.shared_d = (double *)scratch("mg_shared", sizeof(double) * 4);
-  A.out_i = (int *)scratch("mg_out_i", sizeof(int) * (MG_MAX + 4));
-  A.out_d = (double *)scratch("mg_out_d", sizeof(double) * 2);
-  if (!A.partial || !A.shared_d || !A.out_i || !A.out_d) return LEPIC_ERR_CUDA;
+  A.out_i = out_i;
+  A.out_d = out_d;
+  if (!A.partial || !A.shared_d) return LEPIC_ERR_CUDA;
   MGArgs *dA = (MGArgs *)scratch("mg_args", sizeof(MGArgs));
   if (!dA) return LEPIC_ERR_CUDA;
   LEPIC_CUDA(cudaMemcpyAsync(dA, &A, sizeof(MGArgs), cudaMemcpyHostToDevice, s));
@@ -649,15 +1099,7 @@ int launch_pdesolver(const Dims &d, const double h[3], double *u, const double *
   int tm = timer_start("pdesolver_f64", s);
   LEPIC_CUDA(cudaLaunchCooperativeKernel(kern, dim3(blocks), dim3(MG_BLOCK), args, 0, s));
   timer_stop(tm, s);
-  int hi[MG_MAX + 4];
-  double hd[2];
-  LEPIC_CUDA(cudaMemcpyAsync(hi, A.out_i, sizeof(hi), cudaMemcpyDeviceToHost, s));
-  LEPIC_CUDA(cudaMemcpyAsync(hd, A.out_d, sizeof(hd), cudaMemcpyDeviceToHost, s));
-  LEPIC_CUDA(cudaStreamSynchronize(s));
-  if (k_out) *k_out = hi[0];
-  if (ktot_out) *ktot_out = hd[0];
-  if (res_out) *res_out = hd[1];
-  return hi[1];
+  return solve_results(out_i, out_d, k_out, ktot_out, res_out, s);
 }
 
 }  // namespace lepic
@@ -793,13 +1235,5 @@ extern "C" int lepic_dev_pdesolver_noalloc(const lepic_grid_t *g, double *u, con
   LEPIC_CUDA(cudaMemcpyAsync(dA, &A, sizeof(MGArgs), cudaMemcpyHostToDevice, s));
   void *args[] = {&dA};
   LEPIC_CUDA(cudaLaunchCooperativeKernel((void *)k_pdesolver<false>, dim3(blocks), dim3(MG_BLOCK), args, 0, s));
-  int hi[MG_MAX + 4];
-  double hd[2];
-  LEPIC_CUDA(cudaMemcpyAsync(hi, A.out_i, sizeof(hi), cudaMemcpyDeviceToHost, s));
-  LEPIC_CUDA(cudaMemcpyAsync(hd, A.out_d, sizeof(hd), cudaMemcpyDeviceToHost, s));
-  LEPIC_CUDA(cudaStreamSynchronize(s));
-  if (k_out) *k_out = hi[0];
-  if (ktot_out) *ktot_out = hd[0];
-  if (res_out) *res_out = hd[1];
-  return hi[1];
+  return solve_results(A.out_i, A.out_d, k_out, ktot_out, res_out, s);
 }

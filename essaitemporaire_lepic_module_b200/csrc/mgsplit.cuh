@@ -1,0 +1,366 @@
+// Colour-split multigrid levels: the red nodes ((i+j+k) odd) and the black
+// ones of a level live in two arrays of their own, so that a red or black
+// relaxation reads and writes whole cache lines of what it needs (in the
+// natural order each colour is every other value of a line, and both colours'
+// phases move all of them).
+//
+// Node (i, j, k), 0 <= i <= n+2 etc., of colour c (0 red, 1 black) is element
+//   e = (i >> 1) + H (j + N2 k)
+// of that colour's arrays; all nodes of one colour in a row (j, k) have i of
+// one parity s, and in terms of e the six neighbours, all of the other
+// colour, are
+//   west e - 1 + s, east e + s, south/north e -+ H, below/above e -+ H N2.
+// A byte per element holds what the loops ask about its red and its black
+// node (MB_*), the parity s among it, so a relaxation needs no coordinates at all: it runs over the
+// elements of the planes k = 1..n3+1 (whose neighbours are all inside the
+// arrays), every load issued before the byte is looked at, V consecutive
+// elements per thread with vector loads.
+//
+// The red values have two buffers: a red phase reads one and writes the
+// other, so that it can compute the residual of the finished sweep and the
+// next sweep's red values in one pass; when the residual ends the smoothing
+// the written buffer is simply not taken.
+#pragma once
+
+#include <type_traits>
+
+#include "lepic_internal.cuh"
+
+namespace lepic {
+namespace mgs {
+
+// the red node's four bits, the black node's in the upper half (MB(COLOUR, bit))
+enum : unsigned {
+  MB_UPD = 1,      // inside 1..n+1 and not a wall: relaxed
+  MB_PLASMA = 2,   // inside 1..n+1 and bcnd = -1: counted in the residual norm
+  MB_ODD = 4,      // s: parity of i
+  MB_FREE = 8      // not a wall (ghost nodes included): prolonged to
+};
+__host__ __device__ constexpr unsigned MB(int colour, unsigned bit) { return bit << (4 * colour); }
+
+// x / d for 0 <= x < 2^31 by a multiplication (d > 0): with m = ceil(2^p / d),
+// p = 31 + ceil(log2 d), x m exceeds x 2^p / d by x (m d - 2^p) / d, less than
+// 2^p / d
+struct Div {
+  unsigned long long m;
+  int p, d;
+  void set(int dd) {
+    d = dd;
+    int l = 0;
+    while ((1LL << l) < dd) ++l;
+    p = 31 + l;
+    m = ((1ULL << p) + (unsigned)dd - 1) / (unsigned)dd;
+  }
+  __host__ __device__ int div(int x) const { return (int)(((unsigned long long)(unsigned)x * m) >> p); }
+};
+
+template <class T>
+struct Lev {
+  static constexpr int VW = 16 / sizeof(T);   // elements of a 16-byte load
+  int n1, n2, n3;
+  int H, N2, N3;            // row pitch in elements (a multiple of VW), rows per plane, planes
+  int HN, len;              // H N2, elements per colour
+  Div dH, dN2;
+  T aw, an, at, ac;         // ae = aw, as = an, ab = at (Src/mg.h)
+  T rac;                    // 1 / ac, correctly rounded
+  T *red[2], *black;
+  T *b[2];
+  T *rf[2];                 // residual (levels that restrict)
+  unsigned char *m;
+  __host__ __device__ int node(int i, int j, int k) const { return (i >> 1) + H * (j + N2 * k); }
+  __host__ void shape(int a, int bb, int c) {
+    n1 = a;
+    n2 = bb;
+    n3 = c;
+    H = row(a);
+    N2 = n2 + 3;
+    N3 = n3 + 3;
+    HN = H * N2;
+    len = HN * N3;
+    dH.set(H);
+    dN2.set(N2);
+  }
+  static int row(int a) { return (((a + 2) >> 1) + VW) & ~(VW - 1); }
+  // elements of one colour's array of an a x bb x c level
+  static long long elements(int a, int bb, int c) { return (long long)row(a) * (bb + 3) * (c + 3); }
+};
+
+// threads that share a loop
+struct Team {
+  int id, n;
+};
+__device__ __forceinline__ Team grid_team() {
+  return {(int)(blockIdx.x * blockDim.x + threadIdx.x), (int)(gridDim.x * blockDim.x)};
+}
+__device__ __forceinline__ Team block_team() { return {(int)threadIdx.x, (int)blockDim.x}; }
+
+template <class T, int V>
+struct alignas(sizeof(T) * V) Vec {
+  T v[V];
+};
+template <class T, int V>
+__device__ __forceinline__ Vec<T, V> ldv(const T *p) {
+  return *reinterpret_cast<const Vec<T, V> *>(p);
+}
+template <class T, int V>
+__device__ __forceinline__ void stv(T *p, const Vec<T, V> &x) {
+  *reinterpret_cast<Vec<T, V> *>(p) = x;
+}
+
+enum { RED = 0, BLACK = 1 };
+// what a colour's phase does: relax its nodes (ZERO: from 0, not read), add up
+// the residual norm, write the residual out, add the relaxed values to an
+// FP64 solution
+enum { DO_RELAX = 1, DO_RES = 2, DO_RF = 4, DO_ADDU = 8, ZERO = 16 };
+
+// What a phase reads for V consecutive elements: the elements themselves, the
+// six neighbours and the byte (the x neighbours: the other colour's elements
+// at the same place and one more, before or after them).
+template <class T, int V>
+struct Pts {
+  Vec<T, V> x, n, s, t, b, c, r;
+  T e;
+  unsigned m;   // the V bytes, shifted to this colour's bits
+};
+template <class T, int V, int COLOUR, bool SELF = true>
+__device__ __forceinline__ void load_pts(Pts<T, V> &p, int e, int H, int HN, const T *S, const T *O, const T *B,
+                                         const unsigned char *M) {
+  static_assert(V == 2 || V == 4, "");
+  if (V == 2)
+    p.m = *reinterpret_cast<const unsigned short *>(M + e) >> (4 * COLOUR);
+  else
+    p.m = *reinterpret_cast<const unsigned *>(M + e) >> (4 * COLOUR);
+  const T *o = O + e;
+  p.x = ldv<T, V>(o);
+  p.n = ldv<T, V>(o + H);
+  p.s = ldv<T, V>(o - H);
+  p.t = ldv<T, V>(o + HN);
+  p.b = ldv<T, V>(o - HN);
+  if (SELF) p.c = ldv<T, V>(S + e);
+  p.r = ldv<T, V>(B + e);
+  const T lo = o[-1], hi = o[V];
+  p.e = (p.m & MB_ODD) ? hi : lo;
+}
+
+// One colour of a red-black sweep (Src/sors.f90:87-106, 249-267) over the
+// team's elements: reads S (the colour's values) and O (the other colour's),
+// writes D (S itself for black).  DO_RES adds up |residual| over the plasma
+// nodes, with the relaxed value when COLOUR is BLACK (its sweep ends with
+// it) and with the value read when it is RED (the sweep before this one ends
+// with it).  The expressions keep the Fortran order.  (A thread's next
+// elements loaded before the current ones are worked on was slower: twice the
+// registers, spilled at 512 threads.)
+template <class T, int V, int COLOUR, int WHAT>
+__device__ __forceinline__ T colour_phase(const Lev<T> &L, const T *S, T *D, const T *O, T omega, const Team &w,
+                                          T *R = nullptr, double *U = nullptr) {
+  const int e1 = L.HN * (L.n3 + 2), H = L.H, HN = L.HN, step = V * w.n;
+  const T aw = L.aw, an = L.an, at = L.at, ac = L.ac, rac = L.rac;
+  const T *B = L.b[COLOUR];
+  const unsigned char *M = L.m;
+  T acc = T(0);
+#pragma unroll 1
+  for (int e = HN + V * w.id; e < e1; e += step) {
+    Pts<T, V> p;
+    load_pts<T, V, COLOUR, !(WHAT & ZERO)>(p, e, H, HN, S, O, B, M);
+    const bool odd = (p.m & MB_ODD) != 0;
+    Vec<T, V> dv, rv;
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+      const T uw = odd ? p.x.v[v] : (v == 0 ? p.e : p.x.v[v > 0 ? v - 1 : 0]);
+      const T ue = odd ? (v == V - 1 ? p.e : p.x.v[v < V - 1 ? v + 1 : V - 1]) : p.x.v[v];
+      const T u0 = (WHAT & ZERO) ? T(0) : p.c.v[v];
+      const bool upd = (p.m & (MB_UPD << (8 * v))) != 0;
+      T u = u0;
+      if (WHAT & DO_RELAX) {
+        const T tt = p.r.v[v] - aw * uw - an * p.n.v[v] - an * p.s.v[v] - aw * ue - at * p.t.v[v] - at * p.b.v[v];
+        if constexpr (std::is_same_v<T, double>)
+          u = (1.0 - omega) * u0 + div_by(omega * tt, ac, rac);
+        else
+          u = (WHAT & ZERO) ? omega * tt * rac : (1.f - omega) * u0 + omega * tt * rac;
+        u = upd ? u : u0;
+        dv.v[v] = u;
+      }
+      if (WHAT & (DO_RES | DO_RF)) {
+        const T ur = COLOUR == BLACK ? u : u0;
+        const T rij = p.r.v[v] - (aw * uw + an * p.n.v[v] + an * p.s.v[v] + aw * ue + ac * ur + at * p.t.v[v] +
+                                  at * p.b.v[v]);
+        if ((WHAT & DO_RES) && (p.m & (MB_PLASMA << (8 * v)))) acc += rij < T(0) ? -rij : rij;
+        if (WHAT & DO_RF) rv.v[v] = upd ? rij : T(0);
+      }
+    }
+    if (WHAT & DO_RELAX) stv<T, V>(D + e, dv);
+    if (WHAT & DO_RF) stv<T, V>(R + e, rv);
+    if (WHAT & DO_ADDU) {
+#pragma unroll
+      for (int v = 0; v < V; v += 2) {
+        Vec<double, 2> uu = ldv<double, 2>(U + e + v);
+        if (p.m & (MB_UPD << (8 * v))) uu.v[0] += (double)dv.v[v];
+        if (p.m & (MB_UPD << (8 * v + 8))) uu.v[1] += (double)dv.v[v + 1];
+        stv<double, 2>(U + e + v, uu);
+      }
+    }
+  }
+  return acc;
+}
+
+// residual of every node of a colour (Src/mg.f90:808-847, its order of
+// terms), 0 on walls
+template <class T, int V, int COLOUR>
+__device__ __forceinline__ void residual_colour(const Lev<T> &L, const T *S, const T *O, T *R, const Team &w) {
+  const int e1 = L.HN * (L.n3 + 2), H = L.H, HN = L.HN, step = V * w.n;
+  const T aw = L.aw, an = L.an, at = L.at, ac = L.ac;
+  const T *B = L.b[COLOUR];
+  const unsigned char *M = L.m;
+#pragma unroll 1
+  for (int e = HN + V * w.id; e < e1; e += step) {
+    Pts<T, V> p;
+    load_pts<T, V, COLOUR>(p, e, H, HN, S, O, B, M);
+    const bool odd = (p.m & MB_ODD) != 0;
+    Vec<T, V> rv;
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+      const T uw = odd ? p.x.v[v] : (v == 0 ? p.e : p.x.v[v > 0 ? v - 1 : 0]);
+      const T ue = odd ? (v == V - 1 ? p.e : p.x.v[v < V - 1 ? v + 1 : V - 1]) : p.x.v[v];
+      const T r = p.r.v[v] - (aw * uw + aw * ue + an * p.n.v[v] + an * p.s.v[v] + ac * p.c.v[v] + at * p.t.v[v] +
+                              at * p.b.v[v]);
+      rv.v[v] = (p.m & (MB_UPD << (8 * v))) ? r : T(0);
+    }
+    stv<T, V>(R + e, rv);
+  }
+}
+
+// fine node of a coarse one per axis (Src/mg.f90:429-436)
+__device__ __forceinline__ int fine_of(int ic, int ncell_fine) {
+  return ic == ncell_fine / 2 + 2 ? ncell_fine + 2 : (ic == 0 ? 0 : 2 * ic - 1);
+}
+
+// a red node's value after the first red phase of a sweep that starts from 0
+// (the relaxation's own arithmetic with every neighbour 0)
+template <class T>
+__device__ __forceinline__ T first_red(const Lev<T> &L, T b, T omega) {
+  if constexpr (std::is_same_v<T, double>)
+    return (1.0 - omega) * 0.0 + div_by(omega * b, L.ac, L.rac);
+  else
+    return omega * b * L.rac;
+}
+
+// The elements of a level, its whole arrays, over the team's threads:
+// body(e, ii, j, k) for e = ii + H (j + N2 k), of both colours.  (A row per
+// warp needs no division but leaves a third of the lanes idle: a row of 129
+// nodes has 66 elements.)
+template <class T, class F>
+__device__ __forceinline__ void elements(const Lev<T> &L, const Team &w, F &&body) {
+  for (int e = w.id; e < L.len; e += w.n) {
+    const int r = L.dH.div(e), k = L.dN2.div(r), j = r - k * L.N2;
+    body(e, e - r * L.H, j, k);
+  }
+}
+
+// 27-point full weighting (Src/mg.f90:696-702) of F's residual (R, K: its red
+// and black halves, an even / odd number of unit steps from a coarse node's
+// twin) onto C's right-hand side, C's correction cleared; masks: C's node bytes as well
+// (they stay the same for a whole solve).  start: the red values as the first sweep's red
+// phase leaves them (every neighbour is 0 there), so that the sweep begins
+// with its black phase.
+template <class T>
+__device__ __forceinline__ void restrict_to(const Lev<T> &F, const Lev<T> &C, const T *R, const T *K, bool masks,
+                                            bool start, T omega, const Team &w) {
+  const int H = F.H, HN = F.HN;
+  elements(C, w, [&](int e, int ii, int j, int k) {
+    unsigned m = 0;
+    if (masks) {
+      for (int c = 0; c < 2; ++c) {
+        const int s = (c + 1 + j + k) & 1, i = 2 * ii + s;
+        unsigned b = s ? MB_ODD : 0;
+        if (i <= C.n1 + 2) {
+          const int fi = fine_of(i, F.n1), fj = fine_of(j, F.n2), fk = fine_of(k, F.n3);
+          const unsigned fm = F.m[F.node(fi, fj, fk)] >> (4 * ((fi + fj + fk + 1) & 1));
+          b |= fm & MB_FREE;
+          if (i >= 1 && j >= 1 && k >= 1 && i <= C.n1 + 1 && j <= C.n2 + 1 && k <= C.n3 + 1)
+            b |= fm & (MB_UPD | MB_PLASMA);
+        }
+        m |= MB(c, b);
+      }
+      C.m[e] = (unsigned char)m;
+      if (C.rf[RED]) C.rf[RED][e] = T(0);
+      if (C.rf[BLACK]) C.rf[BLACK][e] = T(0);
+    } else {
+      m = C.m[e];
+    }
+    C.black[e] = T(0);
+    // the planes no red phase writes, in both buffers (a ghost that is not a
+    // wall is prolonged to)
+    if (C.red[1] && (masks || k == 0 || k == C.n3 + 2)) C.red[1][e] = T(0);
+    const int q0 = H * ((2 * j - 1) + F.N2 * (2 * k - 1));
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const int i = 2 * ii + ((c + 1 + j + k) & 1);
+      T re = T(0);
+      if (m & MB(c, MB_UPD)) {
+        const int q = (i - 1) + q0;
+        re = (T(8) * R[q] + T(4) * (K[q + 1] + K[q] + K[q + H] + K[q - H] + K[q + HN] + K[q - HN]) +
+              T(2) * (R[q + 1 + H] + R[q + H] + R[q + 1 - H] + R[q - H] + R[q + 1 + HN] + R[q + HN] +
+                      R[q + H + HN] + R[q - H + HN] + R[q + 1 - HN] + R[q - HN] + R[q + H - HN] + R[q - H - HN]) +
+              K[q + 1 + H + HN] + K[q + H + HN] + K[q + 1 - H + HN] + K[q - H + HN] + K[q + 1 + H - HN] +
+              K[q + H - HN] + K[q + 1 - H - HN] + K[q - H - HN]) /
+             T(64);
+      }
+      C.b[c][e] = re;
+      if (c == RED) C.red[0][e] = start && (m & MB(c, MB_UPD)) ? first_red(C, re, omega) : T(0);
+    }
+  });
+}
+
+// Trilinear prolongation (Src/mg.f90:849-939): C's correction added to F's
+// nodes 0..n+1 that are not walls; rF, rC: the current red buffers.  A fine
+// node sits on a coarse one or between two, four or eight (its upper corner
+// first, in the reference's order of terms); which, is the same for a whole
+// row of one colour.  rO: the other red buffer (or null), whose plane k = 0 no
+// red phase writes.
+template <class T>
+__device__ __forceinline__ void prolong_to(const Lev<T> &F, const Lev<T> &C, T *rF, T *rO, const T *rC, const Team &w) {
+  const T *bC = C.black;
+  auto body = [&](int e, int ii, int j, int k) {
+    const unsigned m = F.m[e];
+    if (!(m & (MB(RED, MB_FREE) | MB(BLACK, MB_FREE))) || j > F.n2 + 1 || k > F.n3 + 1) return;
+    const int cj = (j >> 1) + 1, ck = (k >> 1) + 1;     // the upper corner; ci = ii + 1 for both colours
+    const bool y = !(j & 1), z = !(k & 1);              // between coarse nodes along the axis
+    const int a = C.H * (cj + C.N2 * ck);
+    // coarse node (ci - dx, cj - dy, ck - dz): its colour by the sum's parity
+    auto E = [&](int dx, int dy, int dz) -> T {
+      const int ci = ii + 1 - dx;
+      return (((ci + cj - dy + ck - dz) & 1) ? rC : bC)[a + (ci >> 1) - C.H * (dy + C.N2 * dz)];
+    };
+    // the sums along y and z, at the upper x (and, between in x, the lower)
+    const int s = (1 + j + k) & 1;                      // red's parity of i; black's is the other
+    T on, be;                                           // for the colour with i odd / even
+    const T c000 = E(0, 0, 0);
+    if (y && z) {
+      const T c001 = E(0, 0, 1), c011 = E(0, 1, 1), c010 = E(0, 1, 0);
+      on = (c000 + c001 + c011 + c010) / T(4);
+      be = (c000 + c001 + E(1, 0, 1) + E(1, 0, 0) + c010 + c011 + E(1, 1, 1) + E(1, 1, 0)) / T(8);
+    } else if (z) {
+      const T c001 = E(0, 0, 1);
+      on = (c000 + c001) / T(2);
+      be = (c000 + c001 + E(1, 0, 1) + E(1, 0, 0)) / T(4);
+    } else if (y) {
+      const T c010 = E(0, 1, 0);
+      on = (c000 + c010) / T(2);
+      be = (c000 + c010 + E(1, 1, 0) + E(1, 0, 0)) / T(4);
+    } else {
+      on = c000;
+      be = (c000 + E(1, 0, 0)) / T(2);
+    }
+    const bool in0 = 2 * ii <= F.n1 + 1, in1 = 2 * ii + 1 <= F.n1 + 1;   // i even, i odd
+    if ((m & MB(RED, MB_FREE)) && (s ? in1 : in0)) {
+      const T v = rF[e] + (s ? on : be);
+      rF[e] = v;
+      if (rO && k == 0) rO[e] = v;
+    }
+    if ((m & MB(BLACK, MB_FREE)) && (s ? in0 : in1)) F.black[e] = F.black[e] + (s ? be : on);
+  };
+  elements(F, w, body);
+}
+
+}  // namespace mgs
+}  // namespace lepic
