@@ -278,7 +278,7 @@ const char *lepic_build_info(void) {
 namespace lepic {
 namespace {
 // one block: thread 0 waits on an mbarrier phase that nothing completes, at
-// most limit_ns, then records LEPIC_ERR_TIMEOUT as a tile-copy wait does
+// most limit_ns, then records LEPIC_ERR_TIMEOUT
 __global__ void k_wait_selftest(unsigned long long limit_ns, int *err) {
   __shared__ __align__(8) unsigned long long bar;
   const uint32_t b = smem_addr(&bar);

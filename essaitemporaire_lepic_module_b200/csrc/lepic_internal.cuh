@@ -486,8 +486,6 @@ __device__ inline bool mbar_wait_ns(uint32_t bar, uint32_t parity, unsigned long
   return true;
 }
 
-// the library's waits on copies: at most one second
-__device__ inline bool mbar_wait(uint32_t bar, uint32_t parity) { return mbar_wait_ns(bar, parity, 1000000000ull); }
 
 }  // namespace lepic
 

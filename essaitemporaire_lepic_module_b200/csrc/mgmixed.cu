@@ -12,40 +12,28 @@
 // the accumulation of u are FP64, so u converges to the FP64 solution while
 // the V-cycle moves half the bytes.
 //
-// Wall nodes are marked in the FP32 right-hand side itself: r = +inf on a
-// wall or ghost node (never updated; its correction stays 0), so the FP32
-// levels carry no mask arrays.  The coarse masks are the reference's
-// injection (Src/mg.f90:429-436): a coarse node is a wall when the fine node
-// it sits on is one.
-//
-// Grid levels (those too large for one SM's shared memory) are processed in
-// 3D tiles of 32 x 8 x 8 nodes staged in shared memory by the tensor memory
-// accelerator: per tile a block loads the boxes of e and r covering the tile
-// and two halo layers with cp.async.bulk.tensor (double-buffered: the next
-// tile's copy is in flight while the current one is computed, completion on
-// an mbarrier), and works on chip:
-//   sweep      red nodes of tile + 1 halo layer, then black nodes of the tile
-//              (a full red-black sweep per grid phase; the halo's red values
-//              are computed redundantly by the neighbouring tiles);
-//   restrict   the fine residual on tile + 1 halo layer, then the 27-point
-//              weighting onto the coarse nodes whose fine twin lies in the
-//              tile (one grid phase instead of two);
-//   prolong    the coarse correction's box is staged as well and added before
-//              the first post-sweep of the level, in the same phase.
-// The last post-sweep of level 1 also adds the correction to u (FP64).  The
-// coarse levels, from the first one whose arrays fit in shared memory down
-// to the coarsest, run in block 0 alone for each V-cycle, with block
-// barriers only, in the same shared memory.
-//
-// Every wait on a tile copy is bounded (one second); a copy that never
-// completes sets LEPIC_ERR_TIMEOUT in the device error word, the block stops
-// issuing copies and computing, and still meets every grid barrier.
+// All levels are colour-split (mgsplit.cuh): a red or black phase reads and
+// writes only what it needs, 16 bytes per load, and finds walls and parity in
+// one byte per element.  What bounds a solve is the number of grid phases
+// (1.2 us for the barrier alone, 2 to 3 us for a phase of a small level) and,
+// from 128^3 on, the values moved through L2.  A refinement therefore has as
+// few phases as its schedule allows:
+//   * u and b are held as colour-split FP64 copies for the solve, so the FP64
+//     residual is one phase of vector loads, which also does the first
+//     sweep's red phase (from a zero correction it needs no neighbours);
+//     likewise the restriction for the coarser levels;
+//   * the last pre-sweep's black phase writes the black nodes' residual;
+//   * the last sweep of level 1 adds its values to u.
+// Coarse levels that fit the shared memory of one SM run there in block 0.
+// Measured against 32x8x8-node tiles staged by TMA (17 phases of about 22 us a
+// refinement at 128^3): 128^3 warm 1.53 -> 0.69 ms (4 refinements), 256^3 with
+// electrodes cold 40 -> 16.2 ms (18), 48x80x112 warm 0.72 -> 0.40 ms, 32^3
+// 0.38 -> 0.25 ms.
 #include <cooperative_groups.h>
-#include <cuda.h>
 
 #include <cstring>
 
-#include "lepic_internal.cuh"
+#include "mgsplit.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -53,81 +41,58 @@ namespace lepic {
 
 namespace {
 
+using mgs::BLACK;
+using mgs::MB;
+using mgs::MB_FREE;
+using mgs::MB_ODD;
+using mgs::MB_PLASMA;
+using mgs::MB_UPD;
+using mgs::RED;
+using mgs::Team;
+using Lev = mgs::Lev<float>;
+
 constexpr int XM_MAX = 13;      // multigrid levels
-constexpr int GMAX = 6;         // levels in global memory (tiled)
 constexpr int XM_BLOCK = 512;
-constexpr size_t XM_SMEM_COARSE = 160 * 1024;   // budget of the on-chip coarse levels
-
-// tile of updated nodes; the last tile of a row takes the remainder, up to
-// T + 1 nodes (the node n + 1).  TX = 32 puts every fine box on a 16-byte
-// boundary (column 32 t) and every coarse box too (column 16 t); a row of one
-// colour of the tile and its halo (at most 18 nodes) is one warp's.  (A
-// 24-node tile with a row per half-warp was slower at 128^3: 6 tiles per
-// row of 129 nodes instead of 4.)
-constexpr int TX = 32, TY = 8, TZ = 8;
-// staged boxes: the fine box is the tile with two halo layers on each side
-// (one more for a last tile), the coarse box covers what the fine box's
-// nodes interpolate from
-constexpr int BX = TX + 8, BY = TY + 5, BZ = TZ + 5;
-constexpr int CBX = TX / 2 + 4, CBY = TY / 2 + 4, CBZ = TZ / 2 + 4;
-constexpr int BXY = BX * BY;
-constexpr unsigned BOX_BYTES = BX * BY * BZ * 4u;
-constexpr unsigned CBOX_BYTES = CBX * CBY * CBZ * 4u;
-constexpr unsigned BOX_STRIDE = (BOX_BYTES + 127u) / 128u * 128u;
-constexpr unsigned CBOX_STRIDE = (CBOX_BYTES + 127u) / 128u * 128u;
-constexpr unsigned STAGE_BYTES = 2 * BOX_STRIDE + CBOX_STRIDE;  // e box, r box, coarse e box
-constexpr unsigned TILE_SMEM = 2 * STAGE_BYTES + BOX_STRIDE;     // two stages + the residual box
-
-// A level in global memory: FP32 e and r over nodes 0..n+2 per axis, node
-// (i, j, k) at column i + 1 of a row padded to a multiple of 4 floats (so
-// that every tile box starts on a 16-byte boundary, x = 32 t).
-struct GLev {
-  int n1, n2, n3;
-  int P1;              // row pitch, floats
-  int ntx, nty, ntz;   // tiles per axis
-  float aw, an, at, ac;
-  float *e[2];         // the correction, two buffers (a sweep reads one, writes the other)
-  float *r;
-  __host__ __device__ long long g(int i, int j, int k) const {
-    return (long long)(i + 1) + (long long)P1 * (j + (long long)(n2 + 3) * k);
-  }
-  __host__ __device__ long long nn() const { return (long long)P1 * (n2 + 3) * (n3 + 3); }
-};
-
-// A coarse level in block 0's shared memory: nodes 0..n+2, x fastest.
-struct SLev {
-  int n1, n2, n3;
-  int N1, N2;          // n + 3
-  float aw, an, at, ac;
-  float *e, *r, *rf;
-  __device__ int g(int i, int j, int k) const { return i + N1 * (j + N2 * k); }
-};
+constexpr int XV = 4;           // elements per 16-byte load
+constexpr size_t XM_CHIP = 227000;   // shared memory of the levels on chip
 
 struct XArgs {
-  GLev G[GMAX + 2];    // levels 1..min(ls + 1, ng): the grid levels and the exchange level
-  SLev S[XM_MAX + 1];  // levels ls + 1..ng on chip (pointers are shared-memory offsets, set per block)
-  unsigned so_e[XM_MAX + 1], so_r[XM_MAX + 1], so_rf[XM_MAX + 1];
-  int ng, ls;          // levels 1..ls on the grid, ls+1..ng in shared memory
+  Lev L[XM_MAX + 2];          // levels 1..ng; after them level ls + 1 with its arrays on the grid
+  unsigned oc[XM_MAX + 1];    // levels ls+1..ng: byte offset of their arrays on chip
+  unsigned ol;                // and of the level descriptors
+  int ng, ls;                 // levels 1..ls on the grid, ls+1..ng in block 0's shared memory
   int max_refine, nu_fine_pre, nu_fine_post, nu_pre, nu_post, coarse_sweeps;
   float omega;
-  double aw, an, at, ac;  // FP64 finest coefficients (ae = aw, as = an, ab = at)
-  double *u;
+  double aw, an, at, ac;      // FP64 finest coefficients (ae = aw, as = an, ab = at)
+  double *u;                  // the caller's grid arrays
   const double *b;
   const int *bcnd;
+  double *us[2], *bs[2];      // their colour-split copies
   double alpha, eps;
-  double *partial;
+  double *partial;            // [2][gridDim.x]
   int *out_i;      // [0] refinement iterations, [1] status
   double *out_d;   // [0] res/alpha, [1] first res/alpha
-  int *err;        // device error word
 };
 
-// tensor maps of the tile boxes (a __grid_constant__ kernel parameter)
-struct XMaps {
-  CUtensorMap fe[GMAX + 1][2], fr[GMAX + 1];  // fine boxes of e (both buffers) and r, levels 1..ls
-  CUtensorMap ce[GMAX + 2][2];                // coarse boxes of e, levels 2..ls + 1
-};
+extern __shared__ __align__(16) unsigned char xm_smem[];
 
-__device__ __forceinline__ bool wall(float r) { return isinf(r); }
+// level l on the grid / on chip: its descriptor in shared memory
+template <bool GRID>
+__device__ __forceinline__ const Lev &level_of(const XArgs &a, int l) {
+  return reinterpret_cast<const Lev *>(xm_smem + a.ol)[(GRID && l == a.ls + 1 ? a.ng + 1 : l) - 1];
+}
+
+template <bool GRID>
+__device__ __forceinline__ Team team() {
+  return GRID ? mgs::grid_team() : mgs::block_team();
+}
+template <bool GRID>
+__device__ __forceinline__ void barrier(cg::grid_group &grid) {
+  if (GRID)
+    grid.sync();
+  else
+    __syncthreads();
+}
 
 __device__ __forceinline__ double wsum(double v) {
 #pragma unroll
@@ -135,565 +100,257 @@ __device__ __forceinline__ double wsum(double v) {
   return v;
 }
 
-__device__ double bsum(double v, double *sh) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  v = wsum(v);
-  __syncthreads();
-  if (lane == 0) sh[w] = v;
-  __syncthreads();
-  double t = (threadIdx.x < (blockDim.x >> 5)) ? sh[threadIdx.x] : 0.0;
-  if (w == 0) t = wsum(t);
-  if (threadIdx.x == 0) sh[32] = t;
-  __syncthreads();
-  double r = sh[32];
-  __syncthreads();
-  return r;
-}
-
-// deterministic grid-wide sum of one value per thread.  The block partials
-// alternate between two halves of a.partial (parity), so one barrier
-// suffices: a half is rewritten two sums later, after further barriers.
-__device__ double grid_sum(const XArgs &a, double v, int parity, cg::grid_group &grid, double *sh) {
+// deterministic grid-wide sum of one value per thread, ending at a grid
+// barrier.  The block partials alternate between two halves of a.partial
+// (parity), so one barrier suffices: a half is rewritten two sums later.
+__device__ __forceinline__ double grid_sum(const XArgs &a, double v, int parity, cg::grid_group &grid, double *sh) {
   double *part = a.partial + (parity & 1) * gridDim.x;
-  double p = bsum(v, sh);
-  if (threadIdx.x == 0) part[blockIdx.x] = p;
+  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+  v = wsum(v);
+  if (lane == 0) sh[wp] = v;
+  __syncthreads();
+  if (wp == 0) {
+    v = wsum(lane < (int)(blockDim.x >> 5) ? sh[lane] : 0.0);
+    if (lane == 0) part[blockIdx.x] = v;
+  }
   grid.sync();
   double s = 0.0;
-  if (threadIdx.x < 32) {
-    for (int bI = threadIdx.x; bI < (int)gridDim.x; bI += 32) s += part[bI];
-    s = wsum(s);
-    if (threadIdx.x == 0) sh[33] = s;
-  }
-  __syncthreads();
-  s = sh[33];
-  __syncthreads();
-  return s;
-}
-
-// ------------------------------------------------------------ tile copies
-__device__ __forceinline__ void tma_box(uint32_t dst, const CUtensorMap *m, int x, int y, int z, uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], "
-      "[%5];" ::"r"(dst),
-      "l"(reinterpret_cast<unsigned long long>(m)), "r"(x), "r"(y), "r"(z), "r"(bar)
-      : "memory");
-}
-
-// The dynamic shared memory of the kernel: the tile stages (grid phases) or
-// the coarse levels (block 0's coarse cycle).  Box pointers are formed from
-// this symbol so that the compiler addresses them as shared memory.
-extern __shared__ __align__(128) unsigned char xm_smem[];
-
-// The double-buffered tile copies of one block.
-struct Pipe {
-  int base;               // offset of the first 128-byte boundary in xm_smem
-  uint32_t bar[2];        // mbarriers in shared memory
-  unsigned uses[2];       // completed phases per mbarrier
-  bool fail;
-};
-
-enum { K_SWEEP = 1, K_PRO = 2, K_RESTRICT = 4, K_ADDU = 8 };
-
-struct Tile {
-  int tx, ty, tz;
-  int i0, j0, k0;   // node of box index 0 on each axis
-  int w, h, d;      // tile nodes per axis
-};
-
-__device__ __forceinline__ Tile tile_of(const GLev &L, int tau) {
-  Tile t;
-  t.tx = tau % L.ntx;
-  const int q = tau / L.ntx;
-  t.ty = q % L.nty;
-  t.tz = q / L.nty;
-  t.i0 = TX * t.tx - 1;
-  t.j0 = TY * t.ty - 1;
-  t.k0 = TZ * t.tz - 1;
-  t.w = t.tx == L.ntx - 1 ? L.n1 + 1 - TX * t.tx : TX;
-  t.h = t.ty == L.nty - 1 ? L.n2 + 1 - TY * t.ty : TY;
-  t.d = t.tz == L.ntz - 1 ? L.n3 + 1 - TZ * t.tz : TZ;
-  return t;
-}
-
-// thread 0: the copies of tile tau of level l into stage s; ein / cin: the
-// e buffers read (level l, level l + 1)
-__device__ void issue(const XMaps &maps, int l, int kind, const GLev &L, int tau, Pipe &pp, int s, int ein,
-                      int cin) {
-  const Tile t = tile_of(L, tau);
-  const unsigned bytes = 2 * BOX_BYTES + ((kind & K_PRO) ? CBOX_BYTES : 0u);
-  // earlier generic accesses of this stage come before the asynchronous copy
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(pp.bar[s]), "r"(bytes) : "memory");
-  const uint32_t dst = smem_addr(xm_smem + pp.base + s * STAGE_BYTES);
-  tma_box(dst, &maps.fe[l][ein], TX * t.tx, t.j0, t.k0, pp.bar[s]);
-  tma_box(dst + BOX_STRIDE, &maps.fr[l], TX * t.tx, t.j0, t.k0, pp.bar[s]);
-  if (kind & K_PRO)
-    tma_box(dst + 2 * BOX_STRIDE, &maps.ce[l + 1][cin], (TX / 2) * t.tx, (TY / 2) * t.ty - 1, (TZ / 2) * t.tz - 1,
-            pp.bar[s]);
-}
-
-// The rows (y, z) of the region [x0, x0 + nx) x [y0, y0 + ny) x [z0, z0 + nz)
-// dealt to the warps of the block, the lanes along x: body(x, y, z).  The
-// row coordinates advance by the warp count without divisions.
-template <class F>
-__device__ __forceinline__ void box_rows(int x0, int nx, int y0, int ny, int z0, int nz, F &&body) {
-  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  int zz = wp / ny, yy = wp - zz * ny;
-#pragma unroll 2
-  for (; zz < nz;) {
-    const int y = y0 + yy, z = z0 + zz;
-    for (int x = x0 + lane; x < x0 + nx; x += 32) body(x, y, z);
-    yy += nw;
-    while (yy >= ny) {
-      yy -= ny;
-      ++zz;
-    }
-  }
-}
-
-// one red-black colour (red = (i + j + k) odd, Src/sors.f90:87-106) of the box
-// region [x0, x0 + nx) x ... relaxed in place (the Src/sors.f90 update, in
-// FP32): each warp takes a row (at most 32 nodes of one colour: nx <= 64),
-// its rows advance by the warp count.  Every load of a node is issued before
-// its wall test; walls keep their value.
-__device__ __forceinline__ void relax_colour(float *E, const float *R, const Tile &t, int x0, int nx, int y0, int ny,
-                                             int z0, int nz, bool red, float aw, float an, float at, float om,
-                                             float rac) {
-  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const int p0 = (t.i0 + x0 + t.j0 + y0 + t.k0 + z0 + (red ? 1 : 0)) & 1;   // 1: the row's first node is off colour
-  int zz = wp / ny, yy = wp - zz * ny;
-#pragma unroll 2
-  for (; zz < nz;) {
-    const int bx = x0 + ((p0 + yy + zz) & 1) + 2 * lane;
-    const int q = bx + BX * (y0 + yy + BY * (z0 + zz));
-    if (bx < x0 + nx) {
-      const float rv = R[q], e0 = E[q], ew = E[q - 1], ee = E[q + 1], en = E[q + BX], es = E[q - BX],
-                  et = E[q + BXY], eb = E[q - BXY];
-      const float tt = rv - aw * ew - an * en - an * es - aw * ee - at * et - at * eb;
-      const float v = (1.f - om) * e0 + om * tt * rac;
-      if (!wall(rv)) E[q] = v;
-    }
-    yy += nw;
-    while (yy >= ny) {
-      yy -= ny;
-      ++zz;
-    }
-  }
-}
-
-// 27-point full weighting (Src/mg.f90:696-702) of the residual box around q
-__device__ __forceinline__ float weigh27(const float *F, int q) {
-  const int sy = BX, sz = BXY;
-  return (8.f * F[q] + 4.f * (F[q + 1] + F[q - 1] + F[q + sy] + F[q - sy] + F[q + sz] + F[q - sz]) +
-          2.f * (F[q + 1 + sy] + F[q - 1 + sy] + F[q + 1 - sy] + F[q - 1 - sy] + F[q + 1 + sz] + F[q - 1 + sz] +
-                 F[q + sy + sz] + F[q - sy + sz] + F[q + 1 - sz] + F[q - 1 - sz] + F[q + sy - sz] +
-                 F[q - sy - sz]) +
-          F[q + 1 + sy + sz] + F[q - 1 + sy + sz] + F[q + 1 - sy + sz] + F[q - 1 - sy + sz] + F[q + 1 + sy - sz] +
-          F[q - 1 + sy - sz] + F[q + 1 - sy - sz] + F[q - 1 - sy - sz]) *
-         (1.f / 64.f);
-}
-
-// the work of one staged tile (stage s): sweep / prolong+sweep / restrict;
-// eout: the e buffer of level l written
-__device__ void tile_work(const GLev &L, const GLev &C, double *u, float omega, int kind, const Tile &t, int base,
-                          int s, int eout, int cout) {
-  float *E = reinterpret_cast<float *>(xm_smem + base + s * STAGE_BYTES);
-  const float *R = reinterpret_cast<const float *>(xm_smem + base + s * STAGE_BYTES + BOX_STRIDE);
-  const float aw = L.aw, an = L.an, at = L.at, ac = L.ac;
-  const int n1 = L.n1, n2 = L.n2, n3 = L.n3;
-  if (kind & K_PRO) {
-    // trilinear prolongation (Src/mg.f90:849-939) of the coarse box onto
-    // every non-wall node of the fine box inside the grid: a fine node on a
-    // coarse node takes its value, one between coarse nodes their mean
-    const float *CE = reinterpret_cast<const float *>(xm_smem + base + s * STAGE_BYTES + 2 * BOX_STRIDE);
-    const int cx0 = (TX / 2) * t.tx - 1, cy0 = (TY / 2) * t.ty - 1, cz0 = (TZ / 2) * t.tz - 1;
-    box_rows(0, t.w + 4, 0, t.h + 4, 0, t.d + 4, [&](int bx, int by, int bz) {
-      const int i = t.i0 + bx, j = t.j0 + by, k = t.k0 + bz;
-      if (i < 0 || j < 0 || k < 0 || i > n1 + 1 || j > n2 + 1 || k > n3 + 1) return;
-      const int q = bx + BX * (by + BY * bz);
-      if (wall(R[q])) return;
-      const int c = (((i + 1) >> 1) - cx0) + CBX * ((((j + 1) >> 1) - cy0) + CBY * (((k + 1) >> 1) - cz0));
-      // weights of the upper neighbour per axis: 0.5 between coarse nodes, 0 on one
-      const float wx = (i & 1) ? 0.f : 0.5f, wy = (j & 1) ? 0.f : 0.5f, wz = (k & 1) ? 0.f : 0.5f;
-      const float vx = 1.f - wx, vy = 1.f - wy, vz = 1.f - wz;
-      const float s0 = vx * CE[c] + wx * CE[c + 1];
-      const float s1 = vx * CE[c + CBX] + wx * CE[c + 1 + CBX];
-      const float s2 = vx * CE[c + CBX * CBY] + wx * CE[c + 1 + CBX * CBY];
-      const float s3 = vx * CE[c + CBX + CBX * CBY] + wx * CE[c + 1 + CBX + CBX * CBY];
-      E[q] += vz * (vy * s0 + wy * s1) + wz * (vy * s2 + wy * s3);
-    });
-    __syncthreads();
-  }
-  if (kind & K_SWEEP) {
-    const float om = omega, rac = 1.f / ac;
-    // red on the tile and one halo layer, then black on the tile
-    relax_colour(E, R, t, 1, t.w + 2, 1, t.h + 2, 1, t.d + 2, true, aw, an, at, om, rac);
-    __syncthreads();
-    relax_colour(E, R, t, 2, t.w, 2, t.h, 2, t.d, false, aw, an, at, om, rac);
-    __syncthreads();
-  }
-  if (kind & K_RESTRICT) {
-    // residual on the tile and one halo layer (0 on walls), then the coarse
-    // nodes whose fine twin (2I-1, 2J-1, 2K-1) lies in the tile (the first
-    // and last tiles of a row also set the coarse ghost nodes)
-    float *RF = reinterpret_cast<float *>(xm_smem + base + 2 * STAGE_BYTES);
-    box_rows(1, t.w + 2, 1, t.h + 2, 1, t.d + 2, [&](int bx, int by, int bz) {
-      const int q = bx + BX * (by + BY * bz);
-      const float rv = R[q], e0 = E[q], ew = E[q - 1], ee = E[q + 1], en = E[q + BX], es = E[q - BX],
-                  et = E[q + BXY], eb = E[q - BXY];
-      const float v = rv - (aw * ew + aw * ee + an * en + an * es + ac * e0 + at * et + at * eb);
-      RF[q] = wall(rv) ? 0.f : v;
-    });
-    __syncthreads();
-    float *Cr = C.r, *Ce = C.e[cout];
-    const int m1 = C.n1, m2 = C.n2, m3 = C.n3, P1 = C.P1;
-    const int I0 = t.tx == 0 ? 0 : (TX / 2) * t.tx + 1, I1 = t.tx == L.ntx - 1 ? m1 + 2 : (TX / 2) * (t.tx + 1);
-    const int J0 = t.ty == 0 ? 0 : (TY / 2) * t.ty + 1, J1 = t.ty == L.nty - 1 ? m2 + 2 : (TY / 2) * (t.ty + 1);
-    const int K0 = t.tz == 0 ? 0 : (TZ / 2) * t.tz + 1, K1 = t.tz == L.ntz - 1 ? m3 + 2 : (TZ / 2) * (t.tz + 1);
-    box_rows(I0, I1 - I0 + 1, J0, J1 - J0 + 1, K0, K1 - K0 + 1, [&](int I, int J, int K) {
-      float rv = INFINITY;
-      if (I >= 1 && J >= 1 && K >= 1 && I <= m1 + 1 && J <= m2 + 1 && K <= m3 + 1) {
-        const int q = (2 * I - 1 - t.i0) + BX * ((2 * J - 1 - t.j0) + BY * (2 * K - 1 - t.k0));
-        if (!wall(R[q])) rv = weigh27(RF, q);
-      }
-      const long long o = (long long)(I + 1) + (long long)P1 * (J + (long long)(m2 + 3) * K);
-      Cr[o] = rv;
-      Ce[o] = 0.f;
-    });
-  } else {
-    // the tile's correction back to the grid (and, last post-sweep of
-    // level 1, into the FP64 solution)
-    float *Le = L.e[eout];
-    const int P1 = L.P1;
-    const long long U1 = (long long)n1 + 3, U2 = (long long)n2 + 3;
-    box_rows(2, t.w, 2, t.h, 2, t.d, [&](int bx, int by, int bz) {
-      const int q = bx + BX * (by + BY * bz);
-      const int i = t.i0 + bx, j = t.j0 + by, k = t.k0 + bz;
-      const float ev = E[q];
-      Le[(long long)(i + 1) + (long long)P1 * (j + (long long)(n2 + 3) * k)] = ev;
-      if ((kind & K_ADDU) && !wall(R[q])) {
-        double *uq = u + i + U1 * (j + U2 * k);
-        *uq = *uq + (double)ev;
-      }
-    });
-  }
-}
-
-// One pass of `kind` over the tiles of grid level l, ending at a grid
-// barrier.  cur: bit m = the e buffer of level m that holds its correction;
-// a sweep reads it and writes the other one, which becomes current (no
-// block reads what another block of the same phase writes).
-__device__ __noinline__ void tile_pass(const XArgs &a, const XMaps &maps, int l, int kind, Pipe &pp,
-                                       cg::grid_group &grid, unsigned &cur) {
-  // the level descriptors in shared memory for the whole pass
-  __shared__ GLev sL, sC;
-  __shared__ double *su;
-  __shared__ float som;
-  if (threadIdx.x == 0) {
-    sL = a.G[l];
-    if (kind & K_RESTRICT) sC = a.G[l + 1];
-    su = a.u;
-    som = a.omega;
-  }
-  __syncthreads();
-  const GLev &L = sL;
-  const int NT = L.ntx * L.nty * L.ntz;
-  const int ein = (cur >> l) & 1, cin = (cur >> (l + 1)) & 1;
-  const int eout = (kind & K_RESTRICT) ? ein : ein ^ 1;
-  int tau = blockIdx.x;
-  if (tau < NT && threadIdx.x == 0 && !pp.fail) issue(maps, l, kind, L, tau, pp, 0, ein, cin);
-  for (int m = 0; tau < NT; tau += gridDim.x, ++m) {
-    const int s = m & 1;
-    const int nxt = tau + gridDim.x;
-    if (nxt < NT && threadIdx.x == 0 && !pp.fail) issue(maps, l, kind, L, nxt, pp, s ^ 1, ein, cin);
-    __shared__ int ok;
-    if (threadIdx.x == 0) {
-      ok = !pp.fail && mbar_wait(pp.bar[s], pp.uses[s] & 1u);
-      if (!ok && !pp.fail) {
-        pp.fail = true;
-        raise_err(a.err, LEPIC_ERR_TIMEOUT, l);
-      }
-    }
-    __syncthreads();
-    pp.uses[s] += 1;
-    if (ok) tile_work(L, sC, su, som, kind, tile_of(L, tau), pp.base, s, eout, cin);
-    __syncthreads();
-  }
-  if (!(kind & K_RESTRICT)) cur ^= 1u << l;
-  // this phase's stores before the next phase's copies read them
-  asm volatile("fence.proxy.async.global;" ::: "memory");
-  grid.sync();
-}
-
-// ------------------------------------------------------ block 0, on chip
-// flat loop over the nodes (i, j, k) of a box, 32-bit index arithmetic
-template <class F>
-__device__ __forceinline__ void block_box(int i0, int ni, int j0, int nj, int k0, int nk, F &&body) {
-  const int tot = ni * nj * nk;
-  int t = threadIdx.x;
-  if (t >= tot) return;
-  // (i, j, k) of the thread's first element, then stepped by the block size
-  // with carries instead of two integer divisions per element
-  const int row0 = t / ni;
-  int i = t - row0 * ni, k = row0 / nj, j = row0 - k * nj;
-  const int bd = blockDim.x, srow = bd / ni, si = bd - srow * ni;   // bd = srow ni + si
-  const int sk = srow / nj, sj = srow - sk * nj;                    // srow = sk nj + sj
-  for (; t < tot; t += bd) {
-    body(i0 + i, j0 + j, k0 + k);
-    i += si;
-    j += sj;
-    k += sk;
-    if (i >= ni) {
-      i -= ni;
-      ++j;
-    }
-    if (j >= nj) {
-      j -= nj;
-      ++k;
-    }
-  }
-}
-
-// red-black colour start: colour 0 = red ((i+j+k) odd), 1 = black
-// (Src/sors.f90:87-106, 249-267)
-__device__ __forceinline__ int colour_start(int colour, int j, int k) {
-  int is = (colour == 0) ? ((j % 2 == 0) ? 1 : 2) : ((j % 2 == 0) ? 2 : 1);
-  is += (k % 2 == 0) ? 0 : 1;
-  return is > 2 ? 1 : is;
-}
-
-__device__ void b_smooth(const SLev &L, float omega, int nsweep) {
-  const float rac = 1.f / L.ac;
-  const int half = (L.n1 + 2) / 2;
-  const int sy = L.N1, sz = L.N1 * L.N2;
-  for (int s = 0; s < nsweep; ++s) {
-    for (int colour = 0; colour < 2; ++colour) {
-      block_box(0, half, 1, L.n2 + 1, 1, L.n3 + 1, [&](int ii, int j, int k) {
-        const int i = colour_start(colour, j, k) + 2 * ii;
-        if (i > L.n1 + 1) return;
-        const int q = L.g(i, j, k);
-        const float rv = L.r[q];
-        if (wall(rv)) return;
-        const float tt = rv - L.aw * L.e[q - 1] - L.an * L.e[q + sy] - L.an * L.e[q - sy] - L.aw * L.e[q + 1] -
-                         L.at * L.e[q + sz] - L.at * L.e[q - sz];
-        L.e[q] = (1.f - omega) * L.e[q] + omega * tt * rac;
-      });
-      __syncthreads();
-    }
-  }
-}
-
-__device__ void b_restrict(const SLev &F, const SLev &C) {
-  const int sy = F.N1, sz = F.N1 * F.N2;
-  // the residual on every node, 0 on ghosts and walls
-  block_box(0, F.n1 + 3, 0, F.n2 + 3, 0, F.n3 + 3, [&](int i, int j, int k) {
-    const int q = F.g(i, j, k);
-    float v = 0.f;
-    if (i >= 1 && j >= 1 && k >= 1 && i <= F.n1 + 1 && j <= F.n2 + 1 && k <= F.n3 + 1) {
-      const float rv = F.r[q];
-      if (!wall(rv))
-        v = rv - (F.aw * F.e[q - 1] + F.aw * F.e[q + 1] + F.an * F.e[q + sy] + F.an * F.e[q - sy] + F.ac * F.e[q] +
-                  F.at * F.e[q + sz] + F.at * F.e[q - sz]);
-    }
-    F.rf[q] = v;
-  });
-  __syncthreads();
-  block_box(0, C.n1 + 3, 0, C.n2 + 3, 0, C.n3 + 3, [&](int i, int j, int k) {
-    float rv = INFINITY;
-    if (i >= 1 && j >= 1 && k >= 1 && i <= C.n1 + 1 && j <= C.n2 + 1 && k <= C.n3 + 1) {
-      const int q = F.g(2 * i - 1, 2 * j - 1, 2 * k - 1);
-      if (!wall(F.r[q])) {
-        const float *R = F.rf;
-        rv = (8.f * R[q] + 4.f * (R[q + 1] + R[q - 1] + R[q + sy] + R[q - sy] + R[q + sz] + R[q - sz]) +
-              2.f * (R[q + 1 + sy] + R[q - 1 + sy] + R[q + 1 - sy] + R[q - 1 - sy] + R[q + 1 + sz] +
-                     R[q - 1 + sz] + R[q + sy + sz] + R[q - sy + sz] + R[q + 1 - sz] + R[q - 1 - sz] +
-                     R[q + sy - sz] + R[q - sy - sz]) +
-              R[q + 1 + sy + sz] + R[q - 1 + sy + sz] + R[q + 1 - sy + sz] + R[q - 1 - sy + sz] +
-              R[q + 1 + sy - sz] + R[q - 1 + sy - sz] + R[q + 1 - sy - sz] + R[q - 1 - sy - sz]) *
-             (1.f / 64.f);
-      }
-    }
-    const int o = C.g(i, j, k);
-    C.r[o] = rv;
-    C.e[o] = 0.f;
-  });
-  __syncthreads();
-}
-
-// trilinear prolongation of C into F on F's non-wall nodes 0..n+1
-__device__ void b_prolong(const SLev &F, const SLev &C) {
-  block_box(0, F.n1 + 2, 0, F.n2 + 2, 0, F.n3 + 2, [&](int i, int j, int k) {
-    const int q = F.g(i, j, k);
-    if (wall(F.r[q])) return;
-    const int ci = (i + 1) >> 1, cj = (j + 1) >> 1, ck = (k + 1) >> 1;
-    const int ex = (i & 1) ^ 1, ey = (j & 1) ^ 1, ez = (k & 1) ^ 1;
-    const int c0 = C.g(ci, cj, ck);
-    float s = 0.f;
-#pragma unroll
-    for (int dz = 0; dz < 2; ++dz)
-#pragma unroll
-      for (int dy = 0; dy < 2; ++dy)
-#pragma unroll
-        for (int dx = 0; dx < 2; ++dx)
-          if (dx <= ex && dy <= ey && dz <= ez) s += C.e[c0 + dx + C.N1 * (dy + C.N2 * dz)];
-    const int ne = ex + ey + ez;
-    F.e[q] += s * (ne == 0 ? 1.f : (ne == 1 ? 0.5f : (ne == 2 ? 0.25f : 0.125f)));
-  });
-  __syncthreads();
-}
-
-// the coarse levels' view in block 0's shared memory
-__device__ __forceinline__ SLev smem_level(const XArgs &a, int l, unsigned char *sm) {
-  SLev S = a.S[l];
-  S.e = reinterpret_cast<float *>(sm + a.so_e[l]);
-  S.r = reinterpret_cast<float *>(sm + a.so_r[l]);
-  S.rf = reinterpret_cast<float *>(sm + a.so_rf[l]);
-  return S;
-}
-
-// the coarse part of the V-cycle, block 0 only: r of level ls+1 in from the
-// grid (its exchange arrays), e out
-__device__ __noinline__ void coarse_cycle(const XArgs &a, unsigned char *sm) {
-  const int top = a.ls + 1, ng = a.ng;
-  {
-    const GLev &G = a.G[top];
-    const SLev S = smem_level(a, top, sm);
-    block_box(0, S.N1, 0, S.N2, 0, S.n3 + 3, [&](int i, int j, int k) {
-      const int q = S.g(i, j, k);
-      S.r[q] = G.r[G.g(i, j, k)];
-      S.e[q] = 0.f;
-    });
-  }
-  __syncthreads();
-  for (int l = top; l < ng; ++l) {
-    const SLev F = smem_level(a, l, sm), C = smem_level(a, l + 1, sm);
-    b_smooth(F, a.omega, a.nu_pre);
-    b_restrict(F, C);
-  }
-  b_smooth(smem_level(a, ng, sm), a.omega, a.coarse_sweeps);
-  for (int l = ng - 1; l >= top; --l) {
-    const SLev F = smem_level(a, l, sm), C = smem_level(a, l + 1, sm);
-    b_prolong(F, C);
-    b_smooth(F, a.omega, a.nu_post);
-  }
-  {
-    const GLev &G = a.G[top];
-    const SLev S = smem_level(a, top, sm);
-    block_box(0, S.N1, 0, S.N2, 0, S.n3 + 3, [&](int i, int j, int k) { G.e[0][G.g(i, j, k)] = S.e[S.g(i, j, k)]; });
-  }
-  asm volatile("fence.proxy.async.global;" ::: "memory");
+  for (int q = lane; q < (int)gridDim.x; q += 32) s += part[q];   // every warp, in the same order
+  return wsum(s);
 }
 
 // ------------------------------------------------------------ level 1, FP64
-// FP64 residual b - A u of the finest level on its interior nodes, written
-// as the FP32 right-hand side of the V-cycle (+inf on walls), the correction
-// cleared; returns this thread's share of the L1 norm over the plasma nodes
-// (bcnd = -1).  (A flat node index per thread, with two integer divisions per
-// node, made this phase 7 % of the 128^3 solve slower.)
-__device__ __noinline__ double g_residual_f64(const XArgs &a, const GLev &L1, float *e1) {
-  // one grid row (j, k) per warp at a time, the lanes along i: coalesced
-  // loads, no division per node, the arguments in registers
-  const int lane = threadIdx.x & 31;
-  const int gw = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), nw = (int)((gridDim.x * blockDim.x) >> 5);
-  const int ni = L1.n1 + 1, nj = L1.n2 + 1, nk = L1.n3 + 1;
-  const long long sy = L1.n1 + 3, sz = (long long)(L1.n1 + 3) * (L1.n2 + 3);
-  const long long ry = L1.n1 + 2, rz = (long long)(L1.n1 + 2) * (L1.n2 + 2);
-  const double *__restrict__ u = a.u;
-  const double *__restrict__ bb = a.b;
-  const int *__restrict__ bcnd = a.bcnd;
+// One colour of the FP64 residual b - A u, as the FP32 right-hand side of the
+// V-cycle; START: red also takes the first sweep's red phase from a zero
+// correction.  Returns this thread's share of the L1 norm over the plasma
+// nodes (bcnd = -1).
+template <int COLOUR>
+__device__ __forceinline__ double residual_f64(const XArgs &a, const Lev &L, bool start, const Team &w) {
+  const int e1 = L.HN * (L.n3 + 2), H = L.H, HN = L.HN, step = 2 * w.n;
   const double aw = a.aw, an = a.an, at = a.at, ac = a.ac;
-  float *__restrict__ r1 = L1.r;
-  float *__restrict__ e = e1;
+  const double *S = a.us[COLOUR], *O = a.us[COLOUR ^ 1], *B = a.bs[COLOUR];
+  const float om = a.omega;
   double acc = 0.0;
-  for (int row = gw; row < nj * nk; row += nw) {
-    const int k = row / nj + 1, j = row - (k - 1) * nj + 1;
-    const long long w0 = sy * j + sz * k, r0 = ry * j + rz * k, o0 = L1.g(0, j, k);
-#pragma unroll 2
-    for (int i = 1 + lane; i <= ni; i += 32) {
-      const long long w = w0 + i;
-      const int bc = bcnd[w];
-      const double bv = bb[r0 + i], c0 = u[w], uw = u[w - 1], un = u[w + sy], us = u[w - sy], ue = u[w + 1],
-                   ut = u[w + sz], ub = u[w - sz];
-      float rf = INFINITY;
-      if (bc <= 0) {
-        const double rv = bv - (aw * uw + an * un + an * us + aw * ue + ac * c0 + at * ut + at * ub);
-        if (bc == -1) acc += fabs(rv);
-        rf = (float)rv;
-      }
-      r1[o0 + i] = rf;
-      e[o0 + i] = 0.f;
+#pragma unroll 1
+  for (int e = HN + 2 * w.id; e < e1; e += step) {
+    mgs::Pts<double, 2> p;
+    mgs::load_pts<double, 2, COLOUR>(p, e, H, HN, S, O, B, L.m);
+    const bool odd = (p.m & MB_ODD) != 0;
+    mgs::Vec<float, 2> rv, sv;
+#pragma unroll
+    for (int v = 0; v < 2; ++v) {
+      const double uw = odd ? p.x.v[v] : (v == 0 ? p.e : p.x.v[0]);
+      const double ue = odd ? (v == 1 ? p.e : p.x.v[1]) : p.x.v[v];
+      const double r = p.r.v[v] - (aw * uw + an * p.n.v[v] + an * p.s.v[v] + aw * ue + ac * p.c.v[v] +
+                                   at * p.t.v[v] + at * p.b.v[v]);
+      if (p.m & (MB_PLASMA << (8 * v))) acc += fabs(r);
+      const bool upd = (p.m & (MB_UPD << (8 * v))) != 0;
+      rv.v[v] = upd ? (float)r : 0.f;
+      sv.v[v] = upd && start ? mgs::first_red(L, (float)r, om) : 0.f;
     }
+    mgs::stv<float, 2>(L.b[COLOUR] + e, rv);
+    if (COLOUR == RED) mgs::stv<float, 2>(L.red[0] + e, sv);
+    if (COLOUR == BLACK && !start) mgs::stv<float, 2>(L.black + e, sv);
   }
   return acc;
 }
 
-// r = +inf on the ghost nodes of level 1 (never updated, correction 0):
-// one grid row (j, k) per warp, the whole row on the ghost planes j, k = 0,
-// n + 2, else its two end nodes
-__device__ __noinline__ void g_ghosts(const GLev &L) {
-  const int lane = threadIdx.x & 31;
-  const int gw = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), nw = (int)((gridDim.x * blockDim.x) >> 5);
-  const int N1 = L.n1 + 3, N2 = L.n2 + 3, N3 = L.n3 + 3;
-  for (int row = gw; row < N2 * N3; row += nw) {
-    const int k = row / N2, j = row - k * N2;
-    const bool face = j == 0 || k == 0 || j == N2 - 1 || k == N3 - 1;
-    for (int t = lane; t < (face ? N1 : 2); t += 32) {
-      const int i = face ? t : (t == 0 ? 0 : N1 - 1);
-      const long long q = L.g(i, j, k);
-      L.r[q] = INFINITY;
-      L.e[0][q] = 0.f;
-      L.e[1][q] = 0.f;
+// the caller's grids into the split copies, the node bytes and zero ghosts of
+// level 1 (ghost nodes are never prolonged to: their correction stays 0)
+__device__ __noinline__ void split_in(const XArgs &a) {
+  const Lev &L = level_of<true>(a, 1);
+  const long long N1 = L.n1 + 3, R1 = L.n1 + 2, R2 = L.n2 + 2;
+  const int last = L.n1 + 2;
+  mgs::elements(L, mgs::grid_team(), [&](int e, int ii, int j, int k) {
+    // the row's nodes i = 2 ii and 2 ii + 1: one of each colour
+    const long long q = 2 * ii + N1 * (j + (long long)L.N2 * k), qb = 2 * ii + R1 * (j + R2 * (long long)k);
+    const bool jk = j >= 1 && k >= 1 && j <= L.n2 + 1 && k <= L.n3 + 1;
+    const int odd = (j + k + 1) & 1;   // the colour of i odd
+    unsigned m = 0;
+#pragma unroll
+    for (int x = 0; x < 2; ++x) {
+      const int i = 2 * ii + x, c = x ? odd ^ 1 : odd;
+      double u = 0.0, b = 0.0;
+      unsigned bits = x ? MB_ODD : 0;
+      if (i <= last) {
+        u = a.u[q + x];
+        if (jk && i >= 1 && i <= L.n1 + 1) {
+          const int bc = a.bcnd[q + x];
+          b = a.b[qb + x];
+          bits |= (bc <= 0 ? MB_UPD | MB_FREE : 0) | (bc == -1 ? MB_PLASMA : 0);
+        }
+      }
+      m |= MB(c, bits);
+      a.us[c][e] = u;
+      a.bs[c][e] = b;
     }
+    L.m[e] = (unsigned char)m;
+    L.red[0][e] = L.black[e] = 0.f;
+    if (L.rf[RED]) L.rf[RED][e] = L.rf[BLACK][e] = 0.f;
+  });
+}
+__device__ __noinline__ void split_out(const XArgs &a) {
+  const Lev &L = level_of<true>(a, 1);
+  mgs::elements(L, mgs::grid_team(), [&](int e, int ii, int j, int k) {
+    const unsigned m = L.m[e];
+    const int odd = (j + k + 1) & 1;
+    double *u = a.u + 2 * ii + (long long)(L.n1 + 3) * (j + (long long)L.N2 * k);
+#pragma unroll
+    for (int x = 0; x < 2; ++x) {
+      const int c = x ? odd ^ 1 : odd;
+      if (m & MB(c, MB_UPD)) u[x] = a.us[c][e];
+    }
+  });
+}
+
+// ------------------------------------------------------------ FP32 V-cycle
+// nu sweeps of a level.  started: the first red phase is done and black is 0
+// (not written yet); rf: the last black phase also writes the black residual;
+// addu: the last sweep adds its values to u.
+template <bool GRID>
+__device__ __forceinline__ void sweeps(const XArgs &a, const Lev &L, int nu, bool started, bool rf, bool addu,
+                                       cg::grid_group &grid) {
+  using namespace mgs;
+  const Team w = team<GRID>();
+  const float om = a.omega;
+  for (int s = 0; s < nu; ++s) {
+    const bool last = s == nu - 1, add = GRID && addu && last;
+    if (s > 0 || !started) {
+      if (add)
+        colour_phase<float, XV, mgs::RED, DO_RELAX | DO_ADDU>(L, L.red[0], L.red[0], L.black, om, w, nullptr,
+                                                              a.us[mgs::RED]);
+      else
+        colour_phase<float, XV, mgs::RED, DO_RELAX>(L, L.red[0], L.red[0], L.black, om, w);
+      barrier<GRID>(grid);
+    }
+    if (s == 0 && started) {
+      if (last && rf)
+        colour_phase<float, XV, mgs::BLACK, DO_RELAX | DO_RF | ZERO>(L, L.black, L.black, L.red[0], om, w,
+                                                                     L.rf[mgs::BLACK]);
+      else
+        colour_phase<float, XV, mgs::BLACK, DO_RELAX | ZERO>(L, L.black, L.black, L.red[0], om, w);
+    } else if (last && rf) {
+      colour_phase<float, XV, mgs::BLACK, DO_RELAX | DO_RF>(L, L.black, L.black, L.red[0], om, w, L.rf[mgs::BLACK]);
+    } else if (add) {
+      colour_phase<float, XV, mgs::BLACK, DO_RELAX | DO_ADDU>(L, L.black, L.black, L.red[0], om, w, nullptr,
+                                                              a.us[mgs::BLACK]);
+    } else {
+      colour_phase<float, XV, mgs::BLACK, DO_RELAX>(L, L.black, L.black, L.red[0], om, w);
+    }
+    barrier<GRID>(grid);
   }
 }
 
-// u += e on the non-wall nodes of level 1 (when no post-sweep of level 1 did it)
-__device__ __noinline__ void g_add_u(const XArgs &a, const GLev &L1, const float *e1) {
-  const int tid = (int)(blockIdx.x * blockDim.x + threadIdx.x), nth = (int)(gridDim.x * blockDim.x);
-  const int ni = L1.n1 + 1, nj = L1.n2 + 1;
-  const int total = ni * nj * (L1.n3 + 1);
-  for (int t = tid; t < total; t += nth) {
-    const int row = t / ni, i = t - row * ni + 1;
-    const int k = row / nj + 1, j = row - (k - 1) * nj + 1;
-    const long long o = L1.g(i, j, k);
-    if (!wall(L1.r[o])) {
-      double *uq = a.u + i + (long long)(L1.n1 + 3) * (j + (long long)(L1.n2 + 3) * k);
-      *uq = *uq + (double)e1[o];
-    }
-  }
+// the residual of level l (its black half already written when it has been
+// swept) weighted onto level l + 1, whose first red phase is done with it
+template <bool GRID>
+__device__ __forceinline__ void restrict_level(const XArgs &a, int l, bool swept, bool masks, cg::grid_group &grid) {
+  using namespace mgs;
+  const Team w = team<GRID>();
+  const Lev &F = level_of<GRID>(a, l), &C = level_of<GRID>(a, l + 1);
+  residual_colour<float, XV, mgs::RED>(F, F.red[0], F.black, F.rf[mgs::RED], w);
+  if (!swept) residual_colour<float, XV, mgs::BLACK>(F, F.black, F.red[0], F.rf[mgs::BLACK], w);
+  barrier<GRID>(grid);
+  // (a level that is not swept on the way down starts from 0)
+  restrict_to<float>(F, C, F.rf[mgs::RED], F.rf[mgs::BLACK], masks, (l + 1 == a.ng ? a.coarse_sweeps : a.nu_pre) > 0,
+                     a.omega, w);
+  barrier<GRID>(grid);
 }
 
-__global__ void __launch_bounds__(XM_BLOCK, 1)
-    k_refine_mixed(const XArgs *__restrict__ ap, const __grid_constant__ XMaps maps) {
-  cg::grid_group grid = cg::this_grid();
-  const XArgs &a = *ap;
-  __shared__ double sh[40];
-  __shared__ __align__(8) unsigned long long bars[2];
-  const int ng = a.ng, ls = a.ls;
-  Pipe pp;
-  pp.base = (int)((128u - (smem_addr(xm_smem) & 127u)) & 127u);
-  pp.bar[0] = smem_addr(&bars[0]);
-  pp.bar[1] = smem_addr(&bars[1]);
-  pp.uses[0] = pp.uses[1] = 0;
-  pp.fail = false;
-  if (threadIdx.x == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(pp.bar[0]) : "memory");
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(pp.bar[1]) : "memory");
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+// the sweeps of level l on the way down (or the coarsest level's)
+template <bool GRID>
+__device__ __forceinline__ void down_sweeps(const XArgs &a, int l, bool started, cg::grid_group &grid) {
+  const bool coarsest = l == a.ng;
+  const int nu = coarsest ? a.coarse_sweeps : (l == 1 ? a.nu_fine_pre : a.nu_pre);
+  sweeps<GRID>(a, level_of<GRID>(a, l), nu, started, !coarsest, coarsest && a.ng == 1, grid);
+}
+
+// the part of a V-cycle on the levels on chip, by block 0
+__device__ __forceinline__ void chip_cycle(const XArgs &a, bool first, cg::grid_group &grid) {
+  using namespace mgs;
+  const int top = a.ls + 1, ng = a.ng, t0 = threadIdx.x, bd = blockDim.x;
+  const Lev &X = level_of<true>(a, top), &T = level_of<false>(a, top);
+  for (int e = t0; e < T.len; e += bd) {
+    T.b[0][e] = X.b[0][e];
+    T.b[1][e] = X.b[1][e];
+    T.red[0][e] = X.red[0][e];
+    T.black[e] = 0.f;
+    if (first) {
+      T.m[e] = X.m[e];
+      if (T.rf[mgs::RED]) T.rf[mgs::RED][e] = T.rf[mgs::BLACK][e] = 0.f;
+    }
   }
   __syncthreads();
-  unsigned char *smem = xm_smem + pp.base;
-  unsigned cur = 0;   // bit l: the e buffer of level l holding its correction
-  const GLev &L1 = a.G[1];
-  g_ghosts(L1);
-  asm volatile("fence.proxy.async.global;" ::: "memory");
+  const int mid = ng - top;
+  for (int g = 0; g <= 2 * mid; ++g) {
+    const int l = g <= mid ? top + g : ng - (g - mid);
+    if (g <= mid) {
+      down_sweeps<false>(a, l, true, grid);
+      if (g < mid) restrict_level<false>(a, l, a.nu_pre > 0, first, grid);
+    } else {
+      const Lev &F = level_of<false>(a, l), &C = level_of<false>(a, l + 1);
+      prolong_to<float>(F, C, F.red[0], nullptr, C.red[0], block_team());
+      __syncthreads();
+      sweeps<false>(a, F, a.nu_post, false, false, false, grid);
+    }
+  }
+  for (int e = t0; e < T.len; e += bd) {
+    X.red[0][e] = T.red[0][e];
+    X.black[e] = T.black[e];
+  }
+}
+
+// u += e on the non-wall nodes of level 1 (when no sweep of level 1 did it)
+__device__ __noinline__ void add_u(const XArgs &a) {
+  const Lev &L = level_of<true>(a, 1);
+  const Team w = mgs::grid_team();
+  for (int e = w.id; e < L.len; e += w.n) {
+    const unsigned m = L.m[e];
+    if (m & MB(RED, MB_UPD)) a.us[RED][e] += (double)L.red[0][e];
+    if (m & MB(BLACK, MB_UPD)) a.us[BLACK][e] += (double)L.black[e];
+  }
+}
+
+__global__ void __launch_bounds__(XM_BLOCK, 1) k_refine_mixed(const __grid_constant__ XArgs a) {
+  cg::grid_group grid = cg::this_grid();
+  __shared__ double sh[32];
+  const int ng = a.ng, ls = a.ls, down = ls < ng ? ls : ng - 1;   // down: the last grid level restricted from
+  {
+    // the level descriptors in shared memory (read from the kernel's
+    // parameters level by level they cost microseconds of constant-cache
+    // misses per phase), those on chip with their arrays there
+    const int words = (int)(sizeof(Lev) / 4) * (ng + 1);
+    const unsigned *from = reinterpret_cast<const unsigned *>(a.L + 1);
+    for (int q = threadIdx.x; q < words; q += blockDim.x) reinterpret_cast<unsigned *>(xm_smem + a.ol)[q] = from[q];
+    __syncthreads();
+    const int l = ls + 1 + threadIdx.x;
+    if (l <= ng) {
+      Lev &L = const_cast<Lev &>(level_of<false>(a, l));
+      float *p = reinterpret_cast<float *>(xm_smem + a.oc[l]);
+      const int n = L.len;
+      L.red[0] = p;
+      L.black = p + n;
+      L.b[0] = p + 2 * n;
+      L.b[1] = p + 3 * n;
+      if (l < ng) {
+        L.rf[0] = p + 4 * n;
+        L.rf[1] = p + 5 * n;
+      }
+      L.m = reinterpret_cast<unsigned char *>(p + (l < ng ? 6 : 4) * n);
+    }
+    __syncthreads();
+  }
+  split_in(a);
   grid.sync();
   double res = 0.0, res0 = -1.0;
   int it = 0, status = 0;
+  // the residual does the first red phase of level 1, unless there is none or
+  // (one level, one sweep) it is the phase that adds to u
+  const bool start1 = ng == 1 ? a.coarse_sweeps > 1 : a.nu_fine_pre > 0;
   for (;;) {
-    // FP64 residual, FP32 copy as the V-cycle right-hand side, e = 0
-    const double acc = g_residual_f64(a, L1, L1.e[(cur >> 1) & 1]);
-    asm volatile("fence.proxy.async.global;" ::: "memory");
+    const Lev &L1 = level_of<true>(a, 1);
+    double acc = residual_f64<RED>(a, L1, start1, mgs::grid_team());
+    acc += residual_f64<BLACK>(a, L1, start1, mgs::grid_team());
     res = grid_sum(a, acc, it, grid, sh) / a.alpha;
     if (res0 < 0.0) res0 = res;
     if (res < a.eps) break;
@@ -705,97 +362,44 @@ __global__ void __launch_bounds__(XM_BLOCK, 1)
       status = LEPIC_ERR_DIVERGED;
       break;
     }
-    // FP32 V-cycle on the correction: grid levels down (sweeps, fused
-    // residual + restriction), coarse levels on chip, grid levels up (the
-    // first post-sweep prolongs), the last sweep of level 1 adds u += e
-    const int ldown = ls < ng ? ls : ng - 1;   // the last level restricted from
-    for (int l = 1; l <= ldown; ++l) {
-      const int nu = l == 1 ? a.nu_fine_pre : a.nu_pre;
-      for (int s = 0; s < nu; ++s) tile_pass(a, maps, l, K_SWEEP, pp, grid, cur);
-      tile_pass(a, maps, l, K_RESTRICT, pp, grid, cur);
-    }
+    // FP32 V-cycle on the correction: grid levels down, the coarsest level or
+    // the levels on chip, grid levels up
+    const bool first = it == 0;
+    const int mid = down + 1;
     bool added = false;
-    if (ls < ng) {
-      if (blockIdx.x == 0) coarse_cycle(a, smem);
-      grid.sync();
-    } else {
-      // the coarsest level is a grid level: its sweeps (ng = 1: the last one
-      // adds u += e)
-      for (int s = 0; s < a.coarse_sweeps; ++s) {
-        const bool last = ng == 1 && s == a.coarse_sweeps - 1;
-        tile_pass(a, maps, ng, K_SWEEP | (last ? K_ADDU : 0), pp, grid, cur);
-        added = added || last;
-      }
-    }
-    for (int l = (ls < ng ? ls : ng - 1); l >= 1; --l) {
-      const int nu = l == 1 ? a.nu_fine_post : a.nu_post;
-      if (nu == 0) {
-        tile_pass(a, maps, l, K_PRO, pp, grid, cur);
+    for (int g = 1; g <= 2 * down + 1; ++g) {
+      if (g == mid && ls < ng) {
+        if (blockIdx.x == 0) chip_cycle(a, first, grid);
+        grid.sync();
         continue;
       }
-      for (int s = 0; s < nu; ++s) {
-        const bool last = l == 1 && s == nu - 1;
-        tile_pass(a, maps, l, K_SWEEP | (s == 0 ? K_PRO : 0) | (last ? K_ADDU : 0), pp, grid, cur);
-        added = added || last;
+      const int l = g <= mid ? g : 2 * mid - g;
+      if (g <= mid) {
+        down_sweeps<true>(a, l, l > 1 || start1, grid);
+        added = added || (ng == 1 && a.coarse_sweeps > 0);
+        if (g < mid) restrict_level<true>(a, l, (l == 1 ? a.nu_fine_pre : a.nu_pre) > 0, first, grid);
+      } else {
+        const Lev &F = level_of<true>(a, l), &C = level_of<true>(a, l + 1);
+        mgs::prolong_to<float>(F, C, F.red[0], nullptr, C.red[0], mgs::grid_team());
+        grid.sync();
+        const int nu = l == 1 ? a.nu_fine_post : a.nu_post;
+        sweeps<true>(a, F, nu, false, false, l == 1, grid);
+        added = added || (l == 1 && nu > 0);
       }
     }
     if (!added) {
-      g_add_u(a, L1, L1.e[(cur >> 1) & 1]);
+      add_u(a);
       grid.sync();
     }
     ++it;
   }
-  if (pp.fail && threadIdx.x == 0) {
-    // copies possibly in flight: one more bounded wait on each stage
-    mbar_wait(pp.bar[0], pp.uses[0] & 1u);
-    mbar_wait(pp.bar[1], pp.uses[1] & 1u);
-  }
+  split_out(a);
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     a.out_i[0] = it;
     a.out_i[1] = status;
     a.out_d[0] = res;
     a.out_d[1] = res0;
   }
-}
-
-size_t align16(size_t v) { return (v + 15) & ~(size_t)15; }
-
-typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
-                                  const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiledFn encode_tiled() {
-  static EncodeTiledFn fn = nullptr;
-  if (!fn) {
-    void *p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<EncodeTiledFn>(p);
-  }
-  return fn;
-}
-
-// tensor map of array `base` of level L with a box of bx x by x bz floats
-int box_map(CUtensorMap *m, float *base, const GLev &L, unsigned bx, unsigned by, unsigned bz) {
-  EncodeTiledFn fn = encode_tiled();
-  if (!fn) {
-    fprintf(stderr, "lepic_gpu: cuTensorMapEncodeTiled not available\n");
-    return LEPIC_ERR_CUDA;
-  }
-  const cuuint64_t dims[3] = {(cuuint64_t)L.P1, (cuuint64_t)(L.n2 + 3), (cuuint64_t)(L.n3 + 3)};
-  const cuuint64_t strides[2] = {(cuuint64_t)L.P1 * 4, (cuuint64_t)L.P1 * (L.n2 + 3) * 4};
-  const cuuint32_t box[3] = {bx, by, bz};
-  const cuuint32_t es[3] = {1, 1, 1};
-  const CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, base, dims, strides, box, es,
-                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) {
-    fprintf(stderr, "lepic_gpu: cuTensorMapEncodeTiled failed (%d) for a %d x %d x %d level\n", (int)r, L.n1, L.n2,
-            L.n3);
-    return LEPIC_ERR_CUDA;
-  }
-  return LEPIC_OK;
 }
 
 }  // namespace
@@ -829,10 +433,8 @@ int launch_pdesolver_mixed(const Dims &d, const double h[3], double *u, const do
   A.b = b;
   A.bcnd = bcnd;
   A.eps = eps;
-  A.err = c.d_err;
-  // coefficients per level (Src/mg.h) and the coarse levels that fit in
-  // shared memory (level 1 stays on the grid)
-  float co[XM_MAX + 1][4];
+  if (Lev::elements(n[0], n[1], n[2]) >= 1200000000LL) return LEPIC_ERR_UNSUPPORTED;   // 32-bit element numbers
+  // shapes and coefficients per level (Src/mg.h)
   for (int l = 1; l <= ng; ++l) {
     double hl[3];
     for (int q = 0; q < 3; ++q) hl[q] = h[q] * (double)(1 << (l - 1));
@@ -844,102 +446,67 @@ int launch_pdesolver_mixed(const Dims &d, const double h[3], double *u, const do
       A.at = at;
       A.ac = ac;
     }
-    co[l][0] = (float)aw;
-    co[l][1] = (float)an;
-    co[l][2] = (float)at;
-    co[l][3] = (float)ac;
+    Lev &L = A.L[l];
+    L.shape(n[0] >> (l - 1), n[1] >> (l - 1), n[2] >> (l - 1));
+    L.aw = (float)aw;
+    L.an = (float)an;
+    L.at = (float)at;
+    L.ac = (float)ac;
+    L.rac = 1.f / L.ac;
   }
+  // the coarse levels that fit on chip (level 1 stays on the grid): per
+  // element red, black, b of both, on the levels that restrict the residual
+  // of both, one byte
   size_t csm = 0;
   A.ls = ng;
   for (int l = ng; l >= 2; --l) {
-    const size_t nn = (size_t)(n[0] / (1 << (l - 1)) + 3) * (n[1] / (1 << (l - 1)) + 3) * (n[2] / (1 << (l - 1)) + 3);
-    const size_t need = align16(4 * nn) * 3;
-    if (csm + need > XM_SMEM_COARSE) break;
-    A.so_e[l] = (unsigned)csm;
-    A.so_r[l] = (unsigned)(csm + align16(4 * nn));
-    A.so_rf[l] = (unsigned)(csm + 2 * align16(4 * nn));
+    const size_t need = ((size_t)A.L[l].len * (4 * (l < ng ? 6 : 4) + 1) + 15) & ~(size_t)15;
+    if (csm + need > XM_CHIP) break;
+    A.oc[l] = (unsigned)csm;
     csm += need;
     A.ls = l - 1;
   }
-  if (A.ls == ng) csm = 0;
-  const int ngl = A.ls < ng ? A.ls + 1 : ng;   // levels with global arrays
-  if (A.ls > GMAX) {
-    fprintf(stderr, "lepic_gpu: mixed solve: %d grid levels (at most %d)\n", A.ls, GMAX);
-    return LEPIC_ERR_UNSUPPORTED;
-  }
+  A.ol = (unsigned)csm;
+  csm += sizeof(Lev) * (ng + 1);
+  if (A.ls < ng) A.L[ng + 1] = A.L[A.ls + 1];
   char nm[32];
-  for (int l = 1; l <= ng; ++l) {
-    const int m1 = n[0] >> (l - 1), m2 = n[1] >> (l - 1), m3 = n[2] >> (l - 1);
-    if (l <= ngl) {
-      GLev &L = A.G[l];
-      L.n1 = m1;
-      L.n2 = m2;
-      L.n3 = m3;
-      L.P1 = (m1 + 4 + 3) & ~3;
-      L.ntx = (m1 + TX - 1) / TX;
-      L.nty = (m2 + TY - 1) / TY;
-      L.ntz = (m3 + TZ - 1) / TZ;
-      L.aw = co[l][0];
-      L.an = co[l][1];
-      L.at = co[l][2];
-      L.ac = co[l][3];
-      for (int q = 0; q < 2; ++q) {
-        snprintf(nm, sizeof nm, "xm_e%d_%d", l, q);
-        L.e[q] = (float *)scratch(nm, sizeof(float) * (size_t)L.nn());
-        if (!L.e[q]) return LEPIC_ERR_CUDA;
-        // the nodes a sweep never writes (ghosts; walls stay at the 0 the
-        // residual or the restriction gave them) hold 0 in both buffers
-        LEPIC_CUDA(cudaMemsetAsync(L.e[q], 0, sizeof(float) * (size_t)L.nn(), s));
-      }
-      snprintf(nm, sizeof nm, "xm_r%d", l);
-      L.r = (float *)scratch(nm, sizeof(float) * (size_t)L.nn());
-      if (!L.r) return LEPIC_ERR_CUDA;
+  for (int l = 1; l <= A.ls + 1 && l <= ng; ++l) {
+    Lev &L = A.L[l <= A.ls ? l : ng + 1];
+    const size_t len = (size_t)L.len;
+    const bool restricts = l <= A.ls && l < ng;
+    const int halves = restricts ? 6 : 4;
+    snprintf(nm, sizeof nm, "xm_%d", l);
+    float *p = (float *)scratch(nm, (sizeof(float) * halves + 1) * len);
+    if (!p) return LEPIC_ERR_CUDA;
+    L.red[0] = p;
+    L.black = p + len;
+    L.b[0] = p + 2 * len;
+    L.b[1] = p + 3 * len;
+    if (restricts) {
+      L.rf[0] = p + 4 * len;
+      L.rf[1] = p + 5 * len;
     }
-    if (l > A.ls) {
-      SLev &S = A.S[l];
-      S.n1 = m1;
-      S.n2 = m2;
-      S.n3 = m3;
-      S.N1 = m1 + 3;
-      S.N2 = m2 + 3;
-      S.aw = co[l][0];
-      S.an = co[l][1];
-      S.at = co[l][2];
-      S.ac = co[l][3];
-    }
+    L.m = reinterpret_cast<unsigned char *>(p + halves * len);
   }
-  XMaps M;
-  memset(&M, 0, sizeof(M));
-  for (int l = 1; l <= ngl; ++l) {
-    const GLev &L = A.G[l];
-    if (l <= A.ls) {
-      int rc = box_map(&M.fe[l][0], L.e[0], L, BX, BY, BZ);
-      if (!rc) rc = box_map(&M.fe[l][1], L.e[1], L, BX, BY, BZ);
-      if (!rc) rc = box_map(&M.fr[l], L.r, L, BX, BY, BZ);
-      if (rc) return rc;
-    }
-    if (l >= 2) {
-      int rc = box_map(&M.ce[l][0], L.e[0], L, CBX, CBY, CBZ);
-      if (!rc) rc = box_map(&M.ce[l][1], L.e[1], L, CBX, CBY, CBZ);
-      if (rc) return rc;
+  {
+    const size_t len = (size_t)A.L[1].len;
+    double *p = (double *)scratch("xm_f64", sizeof(double) * 4 * len);
+    if (!p) return LEPIC_ERR_CUDA;
+    for (int q = 0; q < 2; ++q) {
+      A.us[q] = p + q * len;
+      A.bs[q] = p + (2 + q) * len;
     }
   }
   A.alpha = fabs((double)((n[0] + 1) * (n[1] + 1) * (n[2] + 1)) * A.ac) * 1.0;
-  const size_t smem = (csm > TILE_SMEM ? csm : TILE_SMEM) + 128;
-  LEPIC_CUDA(cudaFuncSetAttribute(k_refine_mixed, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  int occ = 0;
-  LEPIC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_refine_mixed, XM_BLOCK, smem));
-  if (occ < 1) return LEPIC_ERR_CUDA;
+  LEPIC_CUDA(cudaFuncSetAttribute(k_refine_mixed, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csm));
   const int blocks = c.sms;
   A.partial = (double *)scratch("xm_partial", sizeof(double) * 2 * blocks);
   A.out_i = (int *)scratch("xm_out_i", sizeof(int) * 4);
   A.out_d = (double *)scratch("xm_out_d", sizeof(double) * 2);
-  XArgs *dA = (XArgs *)scratch("xm_args", sizeof(XArgs));
-  if (!A.partial || !A.out_i || !A.out_d || !dA) return LEPIC_ERR_CUDA;
-  LEPIC_CUDA(cudaMemcpyAsync(dA, &A, sizeof(XArgs), cudaMemcpyHostToDevice, s));
-  void *args[] = {&dA, &M};
+  if (!A.partial || !A.out_i || !A.out_d) return LEPIC_ERR_CUDA;
+  void *args[] = {&A};
   int tm = timer_start("pdesolver_mixed", s);
-  LEPIC_CUDA(cudaLaunchCooperativeKernel((void *)k_refine_mixed, dim3(blocks), dim3(XM_BLOCK), args, smem, s));
+  LEPIC_CUDA(cudaLaunchCooperativeKernel((void *)k_refine_mixed, dim3(blocks), dim3(XM_BLOCK), args, csm, s));
   timer_stop(tm, s);
   if (!iters && !res_out) {
     // no wait: the solve's status goes to the device error word
@@ -954,7 +521,6 @@ int launch_pdesolver_mixed(const Dims &d, const double h[3], double *u, const do
   LEPIC_CUDA(cudaStreamSynchronize(s));
   if (iters) *iters = hi[0];
   if (res_out) *res_out = hd[0];
-  // a copy that timed out stays in the device error word (lepic_dev_check)
   return hi[1];
 }
 

@@ -51,8 +51,7 @@ extern "C" {
 #define LEPIC_ERR_NOT_CONVERGED 23 /* iteration cap reached                      */
 #define LEPIC_ERR_SCRATCH_LIMIT 24 /* grid too large for the static scratch of
                                       lepic_dev_pdesolver_noalloc               */
-#define LEPIC_ERR_TIMEOUT 25       /* a bounded device wait ran out (a tile copy
-                                      that never completed)                     */
+#define LEPIC_ERR_TIMEOUT 25       /* a bounded device wait ran out              */
 
 /* ------------------------------------------------------------------------ */
 /* Fortran COMMON blocks of Src/particle_info.h:53-70 and Src/constants.h,   */
@@ -784,8 +783,7 @@ int lepic_dev_check_async(void *stream, int *host);
 /* The failure path of the bounded device waits, for tests: one block whose
  * first thread waits on an mbarrier phase that nothing completes, at most
  * limit_ns (0 < limit_ns <= 2e9) nanoseconds of %globaltimer, then records
- * LEPIC_ERR_TIMEOUT in the device error word as the library's tile-copy
- * waits do when a copy never lands; the context stays usable.  Returns the
+ * LEPIC_ERR_TIMEOUT in the device error word; the context stays usable.  Returns the
  * launch status; the recorded one is read with lepic_dev_check.  No
  * counterpart in the reference. */
 int lepic_dev_wait_selftest(long long limit_ns, void *stream);

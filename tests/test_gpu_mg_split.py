@@ -59,3 +59,42 @@ def test_split_equals_general_kernel(n, ng, walls):
         assert a[:3] == b[:3]
         assert abs(a[3] - b[3]) <= 1e-11 * abs(b[3])     # the norm is summed in another order
         assert np.array_equal(a[4], b[4])
+
+
+@pytest.mark.parametrize("n,ng", [((9, 7, 6), 1), ((10, 14, 18), 2), ((24, 32, 40), 4), ((72, 40, 56), 4)])
+@pytest.mark.parametrize("nu", [(1, 3, 2, 2, 4), (0, 3, 0, 2, 1), (2, 1, 1, 1, 8), (1, 0, 2, 0, 4)])
+def test_mixed_schedules_reach_the_fp64_solution(n, ng, nu):
+    """FP32 cycles of any schedule (sweeps before and after on the finest and
+    on the coarser levels, on the coarsest; 0 among them) in FP64 refinement:
+    the same potential as the FP64 multigrid, both to a residual of 1e-11 of
+    the first one, from which phi is off by less than 1e-6."""
+    import torch
+    from essaitemporaire_lepic_module_b200 import config
+    from essaitemporaire_lepic_module_b200._lib import LepicGrid, lib, phys_struct
+
+    st = config.build("box16")
+    rng = np.random.default_rng(n[0])
+    shape = (n[2] + 3, n[1] + 3, n[0] + 3)
+    bc = np.ones(shape, dtype=np.int32)
+    bc[2:-2, 2:-2, 2:-2] = -1
+    bc[n[2] // 2, n[1] // 2, n[0] // 2:n[0] // 2 + 2] = 2
+    phi0 = np.where(bc == 2, 5.0, np.where(bc == 1, 1.0, 0.0))
+    dev = torch.device("cuda")
+    bct = torch.as_tensor(bc, device=dev)
+    rt = torch.as_tensor(rng.normal(size=tuple(v - 1 for v in shape)) * 1e-5, device=dev)
+    grid = LepicGrid()
+    for a in range(3):
+        grid.n[a], grid.h[a] = n[a], 1.0e-4
+    grid.bcnd = bct.data_ptr()
+    P = phys_struct(st)
+    s = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    a, b = (torch.as_tensor(phi0, device=dev).clone() for _ in range(2))
+    it, res, k, kt = C.c_int(0), C.c_double(0), C.c_int(0), C.c_double(0)
+    rc = lib().lepic_dev_pdesolver_mixed(C.byref(grid), C.c_void_p(a.data_ptr()), C.c_void_p(rt.data_ptr()), 1e-12,
+                                         1.3, ng, C.byref(P), 2000, *nu, C.byref(it), C.byref(res), s)
+    assert rc == 0 and res.value < 1e-12
+    rc = lib().lepic_dev_pdesolver(C.byref(grid), C.c_void_p(b.data_ptr()), C.c_void_p(rt.data_ptr()), 2000, 1e-12,
+                                   1.4, ng, C.byref(P), C.byref(k), C.byref(kt), C.byref(res), s)
+    assert rc == 0
+    assert float((a - b).abs().max()) <= 1e-6 * float(b.abs().max())
+    assert bool((a[bct > 0] == torch.as_tensor(phi0, device=dev)[bct > 0]).all())
