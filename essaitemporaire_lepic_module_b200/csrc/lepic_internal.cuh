@@ -425,6 +425,51 @@ __device__ __forceinline__ bool warp_run_sum(long long key, T (&v)[NV]) {
   return head && key >= 0;
 }
 
+// The distinct keys of a warp's lanes and which lanes have them, in shared
+// memory (one WarpCells per warp).  Returns how many there are (lanes with key
+// -1 have none).  All 32 lanes must call this; the caller's __syncwarp() comes
+// before warp_cell_sums reads it.
+struct WarpCells {
+  long long key[32];
+  unsigned lanes[32];
+};
+__device__ __forceinline__ int warp_cells(long long key, bool wide, WarpCells &S, int *rank = nullptr) {
+  const unsigned full = 0xffffffffu, lt = run_lanemask_le() >> 1;
+  // keys differ in their low 32 bits unless there are more than 2^32 (wide)
+  unsigned m = __match_any_sync(full, (unsigned)key);
+  if (wide) m &= __match_any_sync(full, (unsigned)(key >> 32));
+  const bool lead = key >= 0 && (m & lt) == 0;
+  const unsigned leads = __ballot_sync(full, lead);
+  const int r = lead ? __popc(leads & lt) : -1;
+  if (lead) {
+    S.key[r] = key;
+    S.lanes[r] = m;
+  }
+  if (rank) *rank = r;   // the lane's place in the list when it stands for its key, else -1
+  return __popc(leads);
+}
+// add(r, q, sum over the r-th key's lanes of val(lane, q)) for every key and
+// q < NV: each lane of the warp takes one (key, q) pair at a time, the lanes
+// added up in order.  Particles sorted by cell some steps ago: a warp's
+// particles lie in a few cells, but no longer in runs, so that sums over runs
+// leave most of them to atomics of their own.
+template <int NV, class Val, class Add>
+__device__ __forceinline__ void warp_cell_sums(int ncells, const WarpCells &S, Val val, Add add) {
+  for (int t = threadIdx.x & 31; t < ncells * NV; t += 32) {
+    const int r = t / NV, q = t - r * NV;
+    decltype(val(0, 0)) s0 = 0, s1 = 0;
+    for (unsigned m = S.lanes[r]; m;) {
+      s0 += val(__ffs(m) - 1, q);
+      m &= m - 1;
+      if (m) {
+        s1 += val(__ffs(m) - 1, q);
+        m &= m - 1;
+      }
+    }
+    add(r, q, s0 + s1);
+  }
+}
+
 // ------------------------------------------------------------ exact division
 // a / b from y = RN(1/b), correctly rounded (Markstein, "Computation of
 // elementary functions on the IBM RISC System/6000 processor", IBM J. Res.
@@ -439,6 +484,13 @@ __device__ __forceinline__ double div_by(double a, double b, double y) {
   const double q0 = a * y;
   const double q1 = __fma_rn(__fma_rn(-b, q0, a), y, q0);
   return __fma_rn(__fma_rn(-b, q1, a), y, q1);
+}
+
+// a / b from y = RN(1/b) for a position a: one beyond div_by's
+// range is far outside any grid, and only its cell, clamped by the caller,
+// matters
+__device__ __forceinline__ double quot(double a, double b, double y) {
+  return fabs(a) < 1e200 ? div_by(a, b, y) : a * y;
 }
 
 // ------------------------------------------------ async copies and mbarriers
