@@ -41,7 +41,7 @@ __device__ __forceinline__ unsigned lanemask_lt() {
 }
 
 // what a warp needs to sum its particles' weights per cell
-struct WarpSums {
+struct alignas(16) WarpSums {
   double w[32][10];      // the lanes' eight weights (rows of 80 bytes: no bank conflicts between their stores)
   WarpCells cells;
 };
