@@ -433,19 +433,18 @@ struct WarpCells {
   long long key[32];
   unsigned lanes[32];
 };
-__device__ __forceinline__ int warp_cells(long long key, bool wide, WarpCells &S, int *rank = nullptr) {
+__device__ __forceinline__ int warp_cells(long long key, bool wide, WarpCells &S) {
   const unsigned full = 0xffffffffu, lt = run_lanemask_le() >> 1;
   // keys differ in their low 32 bits unless there are more than 2^32 (wide)
   unsigned m = __match_any_sync(full, (unsigned)key);
   if (wide) m &= __match_any_sync(full, (unsigned)(key >> 32));
   const bool lead = key >= 0 && (m & lt) == 0;
   const unsigned leads = __ballot_sync(full, lead);
-  const int r = lead ? __popc(leads & lt) : -1;
   if (lead) {
+    const int r = __popc(leads & lt);
     S.key[r] = key;
     S.lanes[r] = m;
   }
-  if (rank) *rank = r;   // the lane's place in the list when it stands for its key, else -1
   return __popc(leads);
 }
 // add(r, q, sum over the r-th key's lanes of val(lane, q)) for every key and
