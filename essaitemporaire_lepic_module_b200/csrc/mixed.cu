@@ -802,16 +802,40 @@ __global__ void k_tile_offsets(const int *__restrict__ off, int ntiles, int *__r
   if (t <= ntiles) tile_off[t] = off[(long long)t * (TC * TC * TC)];
 }
 
-// Scatter of the counting sort, one block per chunk of SC_N consecutive
-// particles.  The block groups its particles by key in shared memory (open
-// addressing on the key, the per-key count giving each particle its rank),
-// reserves one range per distinct key with a single atomic on that key's
-// cursor, stages the particles in key order and writes them out so that
-// consecutive threads store consecutive slots of a key's range.
+// The sort's chunks: SC_N consecutive particles per block, counted per key in
+// a shared-memory table (open addressing on the key).
 constexpr int SC_T = 256, SC_U = 4, SC_N = SC_T * SC_U, SC_H = 1024, SC_HBITS = 10;
 constexpr size_t SC_SMEM = sizeof(int) * (4 * SC_H + 2 * SC_N) + sizeof(float) * 6 * SC_N;
 static_assert(SC_H >= SC_N, "the table holds every distinct key of a chunk");
 
+// The lanes' keys (-1: none) counted in the table: each lane's slot and its
+// rank among the block's particles of its key so far.  Neighbouring particles
+// share their cell, and atomics of one warp on one word are serialised, so
+// the lanes of a key are found first and one of them counts for all.  At most
+// SC_N distinct keys per chunk: a free or matching slot exists.
+__device__ __forceinline__ void table_add(int key, int *hkey, int *hcnt, int &slot, int &rank) {
+  const unsigned full = 0xffffffffu;
+  const unsigned same = __match_any_sync(full, key);
+  const int lead = __ffs(same) - 1;
+  int h = 0, base = 0;
+  if (key >= 0 && lead == (int)(threadIdx.x & 31)) {
+    h = (int)(((unsigned)key * 2654435761u) >> (32 - SC_HBITS));
+    for (int probe = 0; probe < SC_H; ++probe) {
+      const int prev = atomicCAS(&hkey[h], -1, key);
+      if (prev == -1 || prev == key) break;
+      h = (h + 1) & (SC_H - 1);
+    }
+    base = atomicAdd(&hcnt[h], __popc(same));
+  }
+  slot = __shfl_sync(full, h, lead);
+  rank = __shfl_sync(full, base, lead) + __popc(same & lmask_lt());
+}
+
+// Scatter of the counting sort.  The block groups its particles by key (the
+// per-key count giving each particle its rank), reserves one range per
+// distinct key with a single atomic on that key's cursor, stages the
+// particles in key order and writes them out so that consecutive threads
+// store consecutive slots of a key's range.
 __global__ void __launch_bounds__(SC_T, 4) k_msort_scatter(const int *__restrict__ cell, const float *__restrict__ p,
                                                            int *__restrict__ cell_o, float *__restrict__ p_o,
                                                            long long cap, const int *__restrict__ count, int ntx,
@@ -844,21 +868,9 @@ __global__ void __launch_bounds__(SC_T, 4) k_msort_scatter(const int *__restrict
   }
 #pragma unroll
   for (int u = 0; u < SC_U; ++u) {
-    const long long idx = c0 + u * SC_T + t;
-    slot[u] = -1;
-    rank[u] = 0;
-    if (idx < N) {
-      const int key = tile_key(cc[u], ntx, nty);
-      unsigned h = ((unsigned)key * 2654435761u) >> (32 - SC_HBITS);
-      // at most SC_N distinct keys per chunk: a free or matching slot exists
-      for (int probe = 0; probe < SC_H; ++probe) {
-        const int prev = atomicCAS(&hkey[h], -1, key);
-        if (prev == -1 || prev == key) break;
-        h = (h + 1) & (SC_H - 1);
-      }
-      slot[u] = (int)h;
-      rank[u] = atomicAdd(&hcnt[h], 1);
-    }
+    const bool in = c0 + u * SC_T + t < N;
+    table_add(in ? tile_key(cc[u], ntx, nty) : -1, hkey, hcnt, slot[u], rank[u]);
+    if (!in) slot[u] = -1;
   }
   __syncthreads();
   {
@@ -909,10 +921,8 @@ __global__ void __launch_bounds__(SC_T, 4) k_msort_scatter(const int *__restrict
   }
 }
 
-// Counts per key of the counting sort, one block per chunk of SC_N
-// particles: the chunk's keys are counted in a shared-memory table (open
-// addressing) and each distinct key adds its count to the global histogram
-// once, instead of one atomic per warp run.
+// Counts per key of the counting sort: each distinct key of a chunk adds its
+// count to the global histogram once.
 __global__ void __launch_bounds__(SC_T) k_msort_hist(const int *__restrict__ cell, const int *__restrict__ count,
                                                      int ntx, int nty, int *__restrict__ cnt) {
   __shared__ int hkey[SC_H], hcnt[SC_H];
@@ -933,15 +943,8 @@ __global__ void __launch_bounds__(SC_T) k_msort_hist(const int *__restrict__ cel
   __syncthreads();
 #pragma unroll
   for (int u = 0; u < SC_U; ++u) {
-    if (key[u] < 0) continue;
-    const int k = tile_key(key[u], ntx, nty);
-    unsigned h = ((unsigned)k * 2654435761u) >> (32 - SC_HBITS);
-    for (int probe = 0; probe < SC_H; ++probe) {
-      const int prev = atomicCAS(&hkey[h], -1, k);
-      if (prev == -1 || prev == k) break;
-      h = (h + 1) & (SC_H - 1);
-    }
-    atomicAdd(&hcnt[h], 1);
+    int slot, rank;
+    table_add(key[u] < 0 ? -1 : tile_key(key[u], ntx, nty), hkey, hcnt, slot, rank);
   }
   __syncthreads();
   for (int q = t; q < SC_H; q += SC_T)
