@@ -425,6 +425,42 @@ __device__ __forceinline__ bool warp_run_sum(long long key, T (&v)[NV]) {
   return head && key >= 0;
 }
 
+// The losses of a push: [0] energy to the walls, [1] energy of the killed
+// particles, then particles and energy per wall label.  Thousands of lost
+// particles a step adding to three words of one label serialise in L2, so
+// each block adds to one of LOSS_COPIES copies, which the end of the hole
+// filling sums into the caller's array.  One scratch buffer holds them behind
+// the hole filling's counters (one memset clears both).
+constexpr int LOSS_COPIES = 64;
+__host__ __device__ constexpr int loss_words(int ngrid) { return 2 + 2 * (ngrid + 1); }
+inline size_t side_bytes(int ngrid) { return 256 + sizeof(double) * LOSS_COPIES * loss_words(ngrid); }
+__host__ __device__ __forceinline__ double *loss_copies(int *side) { return reinterpret_cast<double *>(side + 64); }
+__device__ __forceinline__ double *my_losses(double *copies, int ngrid) {
+  return copies + (blockIdx.x % LOSS_COPIES) * loss_words(ngrid);
+}
+// The end of the hole filling, by the last block of the kernel that moves the
+// particles: the copies into acc (a warp per word), the new count (which every
+// other block has read).  Every thread of the block calls it.
+__device__ __forceinline__ void finish_push(int *count, int *side, double *acc, int ngrid) {
+  __shared__ bool last;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(&side[4], 1) == (int)gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  const double *copies = loss_copies(side);
+  const int n = loss_words(ngrid), lane = threadIdx.x & 31;
+  for (int q = threadIdx.x >> 5; q < n; q += (int)(blockDim.x >> 5)) {
+    double v = copies[lane * n + q] + copies[(lane + 32) * n + q];
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (lane == 0 && v != 0.0) acc[q] += v;
+  }
+  if (threadIdx.x == 0) *count = *count - side[0];
+}
+static_assert(LOSS_COPIES == 64, "two copies per lane");
+
 // The distinct keys of a warp's lanes and which lanes have them, in shared
 // memory (one WarpCells per warp).  Returns how many there are (lanes with key
 // -1 have none).  All 32 lanes must call this; the caller's __syncwarp() comes

@@ -603,6 +603,7 @@ __global__ void __launch_bounds__(MBK, 3) k_push_tiles(
     const int *__restrict__ count, signed char *__restrict__ flag, const int *__restrict__ tile_off,
     const double *__restrict__ kq, double *__restrict__ np, int *__restrict__ holes, int *__restrict__ nholes,
     double *__restrict__ acc, int *__restrict__ err) {
+  acc = my_losses(acc, c.ngrid);
   constexpr int TN = PushBox::N, TT = PushBox::NN, TH = PushBox::H;
   __shared__ float4 s_E[TT];
   __shared__ unsigned char s_cw[PushBox::CN];
@@ -745,6 +746,7 @@ __global__ void __launch_bounds__(MBK, 3) k_push_deposit_tail(
     const int *__restrict__ count, signed char *__restrict__ flag, const int *__restrict__ tile_off,
     const double *__restrict__ kq, double *__restrict__ np, int *__restrict__ holes, int *__restrict__ nholes,
     double *__restrict__ acc, int *__restrict__ err) {
+  acc = my_losses(acc, c.ngrid);
   const Tile T{nullptr, nullptr, nullptr, 0, 0, 0, nullptr};
   const long long N = *count;
   const long long lo = tile_off ? tile_off[c.ntiles] : 0;
@@ -772,8 +774,8 @@ __global__ void k_fillm_lists(const int *__restrict__ count, const int *__restri
 }
 
 __global__ void k_fillm_move(int *__restrict__ cell, float *__restrict__ p, long long cap,
-                             const int *__restrict__ count, signed char *__restrict__ flag, const int *side,
-                             const int *__restrict__ tailA, const int *__restrict__ holeH) {
+                             int *__restrict__ count, signed char *__restrict__ flag, int *side,
+                             const int *__restrict__ tailA, const int *__restrict__ holeH, double *acc, int ngrid) {
   const int N = *count, L = side[0], Np = N - L, na = side[1];
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < na; t += stride) {
@@ -785,9 +787,8 @@ __global__ void k_fillm_move(int *__restrict__ cell, float *__restrict__ p, long
   }
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < L; t += stride)
     flag[Np + t] = 0;
+  finish_push(count, side, acc, ngrid);
 }
-
-__global__ void k_fillm_count(int *count, const int *side) { *count = *count - side[0]; }
 
 // ---------------------------------------------------------------- sort
 // sort key: tile (x-fastest over tiles) * 512 + cell inside the tile
@@ -1138,9 +1139,10 @@ int launch_push_deposit_mixed(const lepic_grid_t &g, const float *E4, lepic_spec
   snprintf(nm, sizeof nm, "mixed_hh%d", p);
   int *holeH = (int *)scratch(nm, sizeof(int) * cap);
   snprintf(nm, sizeof nm, "mixed_side%d", p);
-  int *side = (int *)scratch(nm, sizeof(int) * 4);
+  int *side = (int *)scratch(nm, side_bytes(ngrid));
   if (!holes || !tailA || !holeH || !side) return LEPIC_ERR_CUDA;
-  LEPIC_CUDA(cudaMemsetAsync(side, 0, sizeof(int) * 4, s));
+  LEPIC_CUDA(cudaMemsetAsync(side, 0, side_bytes(ngrid), s));
+  double *loss = loss_copies(side);
   // B-field map: an FP32 copy made at every call (the map may change
   // between calls; (n_B+3)^3 x 48 B of traffic)
   MixedBMap m;
@@ -1181,7 +1183,7 @@ int launch_push_deposit_mixed(const lepic_grid_t &g, const float *E4, lepic_spec
       LEPIC_CUDA(cudaFuncSetAttribute(k_push_tiles<B, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, STAGE_BYTES));
       k_push_tiles<B, D><<<c.ntiles * PUSH_PARTS, MBK, STAGE_BYTES, s>>>(
           d, c, m, E, g.bcnd, g.cell_wall, sp.cell, sp.p, sp.cap, sp.count, sp.flag_dead, sp.tile_off, g.kq, np,
-          holes, side, acc, ctx().d_err);
+          holes, side, loss, ctx().d_err);
     }
     return LEPIC_OK;
   };
@@ -1211,7 +1213,7 @@ int launch_push_deposit_mixed(const lepic_grid_t &g, const float *E4, lepic_spec
     constexpr bool B = decltype(bmap)::value, D = decltype(die)::value;
     k_push_deposit_tail<B, D><<<(int)tail, MBK, 0, s>>>(d, c, m, E, g.bcnd, g.cell_wall, sp.cell, sp.p, sp.cap,
                                                         sp.count, sp.flag_dead, sp.tile_off, g.kq, np, holes,
-                                                        side, acc, ctx().d_err);
+                                                        side, loss, ctx().d_err);
   };
   if (m.B && die)
     run_tail(std::true_type{}, std::true_type{});
@@ -1226,8 +1228,7 @@ int launch_push_deposit_mixed(const lepic_grid_t &g, const float *E4, lepic_spec
   int t1 = timer_start("fill_holes_mixed", s);
   const int fb = ctx().sms * 2;
   k_fillm_lists<<<fb, 256, 0, s>>>(sp.count, holes, sp.flag_dead, side, tailA, holeH);
-  k_fillm_move<<<fb, 256, 0, s>>>(sp.cell, sp.p, sp.cap, sp.count, sp.flag_dead, side, tailA, holeH);
-  k_fillm_count<<<1, 1, 0, s>>>(sp.count, side);
+  k_fillm_move<<<fb, 256, 0, s>>>(sp.cell, sp.p, sp.cap, sp.count, sp.flag_dead, side, tailA, holeH, acc, ngrid);
   timer_stop(t1, s);
   LEPIC_CUDA(cudaGetLastError());
   return LEPIC_OK;

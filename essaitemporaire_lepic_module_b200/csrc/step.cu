@@ -108,6 +108,7 @@ __global__ void __launch_bounds__(FB) k_push_deposit_f64(
     double *__restrict__ np, int *__restrict__ holes, int *__restrict__ nholes,
     double *__restrict__ acc, int *__restrict__ err) {
   const unsigned full = 0xffffffffu;
+  acc = my_losses(acc, c.ngrid);
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   const int N = *count;
   long long q = -1;  // deposit base node of this lane, -1: nothing to deposit
@@ -252,9 +253,9 @@ __global__ void k_fill_lists(const int *__restrict__ count, const int *__restric
   }
 }
 
-__global__ void k_fill_move(double *__restrict__ p, long long cap, const int *__restrict__ count,
-                            signed char *__restrict__ flag, const int *side, const int *__restrict__ tailA,
-                            const int *__restrict__ holeH) {
+__global__ void k_fill_move(double *__restrict__ p, long long cap, int *__restrict__ count,
+                            signed char *__restrict__ flag, int *side, const int *__restrict__ tailA,
+                            const int *__restrict__ holeH, double *acc, int ngrid) {
   const int N = *count, L = side[0], Np = N - L, na = side[1];
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < na; t += stride) {
@@ -265,9 +266,8 @@ __global__ void k_fill_move(double *__restrict__ p, long long cap, const int *__
   }
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < L; t += stride)
     flag[Np + t] = 0;
+  finish_push(count, side, acc, ngrid);
 }
-
-__global__ void k_fill_count(int *count, const int *side) { *count = *count - side[0]; }
 
 }  // namespace
 
@@ -312,26 +312,26 @@ int launch_push_deposit(const lepic_grid_t &g, const double *Ei, lepic_species_f
   snprintf(nm, sizeof nm, "fused_hh%d", p);
   int *holeH = (int *)scratch(nm, sizeof(int) * cap);
   snprintf(nm, sizeof nm, "fused_side%d", p);
-  int *side = (int *)scratch(nm, sizeof(int) * 4);
+  int *side = (int *)scratch(nm, side_bytes(ngrid));
   if (!holes || !tailA || !holeH || !side) return LEPIC_ERR_CUDA;
-  LEPIC_CUDA(cudaMemsetAsync(side, 0, sizeof(int) * 4, s));
+  LEPIC_CUDA(cudaMemsetAsync(side, 0, side_bytes(ngrid), s));
+  double *loss = loss_copies(side);
   const int nthreads = n_hint > 0 ? n_hint : sp.cap;
   int t0 = timer_start("push_deposit_f64", s);
   if (m.B)
     k_push_deposit_f64<true><<<grid_for(nthreads, FB), FB, 0, s>>>(d, c, m, die, Ei, g.bcnd, g.cell_wall, sp.p,
                                                                    sp.cap, sp.count, sp.flag_dead, g.kq, np,
-                                                                   holes, side, acc_dev, ctx().d_err);
+                                                                   holes, side, loss, ctx().d_err);
   else
     k_push_deposit_f64<false><<<grid_for(nthreads, FB), FB, 0, s>>>(d, c, m, die, Ei, g.bcnd, g.cell_wall, sp.p,
                                                                     sp.cap, sp.count, sp.flag_dead, g.kq, np,
-                                                                    holes, side, acc_dev, ctx().d_err);
+                                                                    holes, side, loss, ctx().d_err);
   timer_stop(t0, s);
   LEPIC_CUDA(cudaGetLastError());
   int t1 = timer_start("fill_holes", s);
   const int fb = ctx().sms * 2;
   k_fill_lists<<<fb, 256, 0, s>>>(sp.count, holes, sp.flag_dead, side, tailA, holeH);
-  k_fill_move<<<fb, 256, 0, s>>>(sp.p, sp.cap, sp.count, sp.flag_dead, side, tailA, holeH);
-  k_fill_count<<<1, 1, 0, s>>>(sp.count, side);
+  k_fill_move<<<fb, 256, 0, s>>>(sp.p, sp.cap, sp.count, sp.flag_dead, side, tailA, holeH, acc_dev, ngrid);
   timer_stop(t1, s);
   LEPIC_CUDA(cudaGetLastError());
   return LEPIC_OK;
