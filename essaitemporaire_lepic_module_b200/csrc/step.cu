@@ -99,9 +99,11 @@ __device__ __forceinline__ void warp_deposit(const Dims &d, long long q, const d
       });
 }
 
-// BMAP: B from the map m (else the uniform c.Bx, c.By, c.Bz)
+// BMAP: B from the map m (else the uniform c.Bx, c.By, c.Bz).  Five blocks per
+// SM: the sums' shared-memory latency wants warps (2.6e7 particles: 1.40 ms at
+// the compiler's own register count, 1.07 with five blocks)
 template <bool BMAP>
-__global__ void __launch_bounds__(FB) k_push_deposit_f64(
+__global__ void __launch_bounds__(FB, 5) k_push_deposit_f64(
     Dims d, FusedConst c, BMapF64 m, Dielectric die, const double *__restrict__ Ei, const int *__restrict__ bcnd,
     const unsigned char *__restrict__ cw, double *__restrict__ p, long long cap,
     const int *__restrict__ count, signed char *__restrict__ flag, const double *__restrict__ kq,
