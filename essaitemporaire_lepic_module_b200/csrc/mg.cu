@@ -741,16 +741,21 @@ __device__ __forceinline__ void chip_cycle(const SPArgs &a, bool first, int *ite
   int cur[MG_MAX + 1];
   const Lev<double> &X = level_of<true>(a, top);
   {
+    // two elements per thread and turn, every load before the first store
     const Lev<double> &L = level_of<false>(a, top);
-    for (int e = t0; e < L.len; e += bd) {
-      L.b[0][e] = X.b[0][e];
-      L.b[1][e] = X.b[1][e];
-      L.red[0][e] = X.red[0][e];   // the first red phase is done
-      L.black[e] = 0.0;
-      if (first || e < L.HN || e >= L.HN * (L.n3 + 2)) L.red[1][e] = 0.0;   // planes no red phase writes
+    for (int e = 2 * t0; e < L.len; e += 2 * bd) {
+      const Vec<double, 2> b0 = ldv<double, 2>(X.b[0] + e), b1 = ldv<double, 2>(X.b[1] + e),
+                           r0 = ldv<double, 2>(X.red[0] + e);   // the first red phase is done
+      const unsigned short m = first ? *reinterpret_cast<const unsigned short *>(X.m + e) : 0;
+      const Vec<double, 2> zero = {{0.0, 0.0}};
+      stv<double, 2>(L.b[0] + e, b0);
+      stv<double, 2>(L.b[1] + e, b1);
+      stv<double, 2>(L.red[0] + e, r0);
+      stv<double, 2>(L.black + e, zero);
+      if (first || e < L.HN || e >= L.HN * (L.n3 + 2)) stv<double, 2>(L.red[1] + e, zero);   // planes no red phase writes
       if (first) {
-        L.m[e] = X.m[e];
-        if (L.rf[BLACK]) L.rf[BLACK][e] = 0.0;
+        *reinterpret_cast<unsigned short *>(L.m + e) = m;
+        if (L.rf[BLACK]) stv<double, 2>(L.rf[BLACK] + e, zero);
       }
     }
     __syncthreads();
@@ -772,9 +777,9 @@ __device__ __forceinline__ void chip_cycle(const SPArgs &a, bool first, int *ite
     if (g < mid) restrict_level<false>(a, l, cur[l], first, grid);
   }
   const Lev<double> &L = level_of<false>(a, top);
-  for (int e = t0; e < L.len; e += bd) {
-    X.red[0][e] = L.red[cur[top]][e];
-    X.black[e] = L.black[e];
+  for (int e = 2 * t0; e < L.len; e += 2 * bd) {
+    stv<double, 2>(X.red[0] + e, ldv<double, 2>(L.red[cur[top]] + e));
+    stv<double, 2>(X.black + e, ldv<double, 2>(L.black + e));
   }
 }
 

@@ -270,14 +270,22 @@ __device__ __forceinline__ void chip_cycle(const XArgs &a, bool first, cg::grid_
   using namespace mgs;
   const int top = a.ls + 1, ng = a.ng, t0 = threadIdx.x, bd = blockDim.x;
   const Lev &X = level_of<true>(a, top), &T = level_of<false>(a, top);
-  for (int e = t0; e < T.len; e += bd) {
-    T.b[0][e] = X.b[0][e];
-    T.b[1][e] = X.b[1][e];
-    T.red[0][e] = X.red[0][e];
-    T.black[e] = 0.f;
+  // four elements per thread and turn, every load before the first store
+  for (int e = XV * t0; e < T.len; e += XV * bd) {
+    const Vec<float, XV> b0 = ldv<float, XV>(X.b[0] + e), b1 = ldv<float, XV>(X.b[1] + e),
+                         r0 = ldv<float, XV>(X.red[0] + e);
+    const unsigned m = first ? *reinterpret_cast<const unsigned *>(X.m + e) : 0u;
+    const Vec<float, XV> zero = {{0.f, 0.f, 0.f, 0.f}};
+    stv<float, XV>(T.b[0] + e, b0);
+    stv<float, XV>(T.b[1] + e, b1);
+    stv<float, XV>(T.red[0] + e, r0);
+    stv<float, XV>(T.black + e, zero);
     if (first) {
-      T.m[e] = X.m[e];
-      if (T.rf[mgs::RED]) T.rf[mgs::RED][e] = T.rf[mgs::BLACK][e] = 0.f;
+      *reinterpret_cast<unsigned *>(T.m + e) = m;
+      if (T.rf[mgs::RED]) {
+        stv<float, XV>(T.rf[mgs::RED] + e, zero);
+        stv<float, XV>(T.rf[mgs::BLACK] + e, zero);
+      }
     }
   }
   __syncthreads();
@@ -294,9 +302,9 @@ __device__ __forceinline__ void chip_cycle(const XArgs &a, bool first, cg::grid_
       sweeps<false>(a, F, a.nu_post, false, false, false, grid);
     }
   }
-  for (int e = t0; e < T.len; e += bd) {
-    X.red[0][e] = T.red[0][e];
-    X.black[e] = T.black[e];
+  for (int e = XV * t0; e < T.len; e += XV * bd) {
+    stv<float, XV>(X.red[0] + e, ldv<float, XV>(T.red[0] + e));
+    stv<float, XV>(X.black + e, ldv<float, XV>(T.black + e));
   }
 }
 

@@ -316,50 +316,68 @@ __device__ __forceinline__ void restrict_to(const Lev<T> &F, const Lev<T> &C, co
 // node sits on a coarse one or between two, four or eight (its upper corner
 // first, in the reference's order of terms); which, is the same for a whole
 // row of one colour.  rO: the other red buffer (or null), whose plane k = 0 no
-// red phase writes.
+// red phase writes.  A thread takes two elements of a row, ii and ii + 1 (ii
+// even): their nodes 2 ii .. 2 ii + 3 lie between the coarse columns ii .. ii + 2.
+// Every load is issued before the bytes are looked at.
 template <class T>
 __device__ __forceinline__ void prolong_to(const Lev<T> &F, const Lev<T> &C, T *rF, T *rO, const T *rC, const Team &w) {
   const T *bC = C.black;
-  auto body = [&](int e, int ii, int j, int k) {
-    const unsigned m = F.m[e];
-    if (!(m & (MB(RED, MB_FREE) | MB(BLACK, MB_FREE))) || j > F.n2 + 1 || k > F.n3 + 1) return;
-    const int cj = (j >> 1) + 1, ck = (k >> 1) + 1;     // the upper corner; ci = ii + 1 for both colours
+  const int H = C.H, HN = C.HN, last = F.n1 + 1;
+#pragma unroll 1
+  for (int e = 2 * w.id; e < F.len; e += 2 * w.n) {
+    const int r = F.dH.div(e), k = F.dN2.div(r), j = r - k * F.N2, ii = e - r * F.H;
+    if (2 * ii > last || j > F.n2 + 1 || k > F.n3 + 1) continue;
+    const unsigned m = *reinterpret_cast<const unsigned short *>(F.m + e);
+    Vec<T, 2> vr = ldv<T, 2>(rF + e), vb = ldv<T, 2>(F.black + e);
+    // the corner (ii + 1, cj, ck) of the first element's even node; the node
+    // one step from another is of the other colour
+    const int cj = (j >> 1) + 1, ck = (k >> 1) + 1;
     const bool y = !(j & 1), z = !(k & 1);              // between coarse nodes along the axis
-    const int a = C.H * (cj + C.N2 * ck);
-    // coarse node (ci - dx, cj - dy, ck - dz): its colour by the sum's parity
-    auto E = [&](int dx, int dy, int dz) -> T {
-      const int ci = ii + 1 - dx;
-      return (((ci + cj - dy + ck - dz) & 1) ? rC : bC)[a + (ci >> 1) - C.H * (dy + C.N2 * dz)];
+    const int u = (ii >> 1) + H * (cj + C.N2 * ck);
+    const bool odd = (ii + 1 + cj + ck) & 1;
+    const T *P = odd ? rC : bC, *Q = odd ? bC : rC;     // the corner's colour and the other
+    // columns ii, ii + 1 and ii + 2 of the up to four coarse rows: element
+    // ii / 2 of Q, ii / 2 of P, ii / 2 + 1 of Q (rows one step away: P and Q
+    // change places)
+    T a0[3], a1[3], a2[3], a3[3];
+    const bool more = 2 * ii + 2 <= last;               // the second element has nodes to prolong to
+    auto row = [&](T (&a)[3], const T *p, const T *q, int at) {
+      a[0] = q[at];
+      a[1] = p[at];
+      a[2] = more ? q[at + 1] : T(0);
     };
-    // the sums along y and z, at the upper x (and, between in x, the lower)
+    row(a0, P, Q, u);
+    if (z) row(a1, Q, P, u - HN);
+    if (y) row(a2, Q, P, u - H);
+    if (y && z) row(a3, P, Q, u - H - HN);
     const int s = (1 + j + k) & 1;                      // red's parity of i; black's is the other
-    T on, be;                                           // for the colour with i odd / even
-    const T c000 = E(0, 0, 0);
-    if (y && z) {
-      const T c001 = E(0, 0, 1), c011 = E(0, 1, 1), c010 = E(0, 1, 0);
-      on = (c000 + c001 + c011 + c010) / T(4);
-      be = (c000 + c001 + E(1, 0, 1) + E(1, 0, 0) + c010 + c011 + E(1, 1, 1) + E(1, 1, 0)) / T(8);
-    } else if (z) {
-      const T c001 = E(0, 0, 1);
-      on = (c000 + c001) / T(2);
-      be = (c000 + c001 + E(1, 0, 1) + E(1, 0, 0)) / T(4);
-    } else if (y) {
-      const T c010 = E(0, 1, 0);
-      on = (c000 + c010) / T(2);
-      be = (c000 + c010 + E(1, 1, 0) + E(1, 0, 0)) / T(4);
-    } else {
-      on = c000;
-      be = (c000 + E(1, 0, 0)) / T(2);
+#pragma unroll
+    for (int v = 0; v < 2; ++v) {
+      // corner column v + 1, the lower column v
+      T on, be;                                         // for the colour with i odd / even
+      if (y && z) {
+        on = (a0[v + 1] + a1[v + 1] + a3[v + 1] + a2[v + 1]) / T(4);
+        be = (a0[v + 1] + a1[v + 1] + a1[v] + a0[v] + a2[v + 1] + a3[v + 1] + a3[v] + a2[v]) / T(8);
+      } else if (z) {
+        on = (a0[v + 1] + a1[v + 1]) / T(2);
+        be = (a0[v + 1] + a1[v + 1] + a1[v] + a0[v]) / T(4);
+      } else if (y) {
+        on = (a0[v + 1] + a2[v + 1]) / T(2);
+        be = (a0[v + 1] + a2[v + 1] + a2[v] + a0[v]) / T(4);
+      } else {
+        on = a0[v + 1];
+        be = (a0[v + 1] + a0[v]) / T(2);
+      }
+      const int i = 2 * (ii + v);
+      const bool in0 = i <= last, in1 = i + 1 <= last;  // i even, i odd
+      const unsigned mv = m >> (8 * v);
+      if ((mv & MB(RED, MB_FREE)) && (s ? in1 : in0)) vr.v[v] = vr.v[v] + (s ? on : be);
+      if ((mv & MB(BLACK, MB_FREE)) && (s ? in0 : in1)) vb.v[v] = vb.v[v] + (s ? be : on);
     }
-    const bool in0 = 2 * ii <= F.n1 + 1, in1 = 2 * ii + 1 <= F.n1 + 1;   // i even, i odd
-    if ((m & MB(RED, MB_FREE)) && (s ? in1 : in0)) {
-      const T v = rF[e] + (s ? on : be);
-      rF[e] = v;
-      if (rO && k == 0) rO[e] = v;
-    }
-    if ((m & MB(BLACK, MB_FREE)) && (s ? in0 : in1)) F.black[e] = F.black[e] + (s ? be : on);
-  };
-  elements(F, w, body);
+    stv<T, 2>(rF + e, vr);
+    stv<T, 2>(F.black + e, vb);
+    if (rO && k == 0) stv<T, 2>(rO + e, vr);
+  }
 }
 
 }  // namespace mgs
