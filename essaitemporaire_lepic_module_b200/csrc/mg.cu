@@ -585,6 +585,7 @@ __global__ void __launch_bounds__(MG_BLOCK) k_pdesolver(const MGArgs *__restrict
 // finest level, barriers and the latency of dependent FP64 operations below.
 // 512 threads: with 768 and 1024 the phases spill (128^3: 4.8 and 5.8 ms).
 constexpr int SP_BLOCK = 512;
+constexpr long long SP_SMALL = 40000;   // elements per colour one cluster solves faster than the grid
 constexpr size_t SP_CHIP = 227000;   // shared memory of the levels on chip: 16^3 and below
 
 struct SPArgs {
@@ -658,9 +659,9 @@ __device__ __forceinline__ double *residual_red(const mgs::Lev<double> &L, int c
 // sweep l - 1 is known after the red phase of sweep l.  Returns the last
 // sweep's residual when need_res, the sweeps done in ksor.  started: the
 // restriction has done the first sweep's red phase.
-template <bool GRID>
+template <bool GRID, class Sync>
 __device__ __forceinline__ double smooth(const SPArgs &a, int level, int &cur, bool first, int dig, bool need_res,
-                                         bool started, cg::grid_group &grid, double *sh, int &ksor) {
+                                         bool started, Sync &grid, double *sh, int &ksor) {
   using namespace mgs;
   const Lev<double> &L = level_of<GRID>(a, level);
   const Team w = GRID ? grid_team() : block_team();
@@ -715,8 +716,8 @@ __device__ __forceinline__ double smooth(const SPArgs &a, int level, int &cur, b
 }
 
 // the residual of a level weighted onto the next one
-template <bool GRID>
-__device__ __forceinline__ void restrict_level(const SPArgs &a, int level, int cur, bool masks, cg::grid_group &grid) {
+template <bool GRID, class Sync>
+__device__ __forceinline__ void restrict_level(const SPArgs &a, int level, int cur, bool masks, Sync &grid) {
   using namespace mgs;
   const Lev<double> &F = level_of<GRID>(a, level), &C = level_of<GRID>(a, level + 1);
   double *R = residual_red(F, cur);
@@ -735,7 +736,8 @@ __device__ __forceinline__ void restrict_level(const SPArgs &a, int level, int c
 }
 
 // the part of a V-cycle on the levels on chip, by block 0
-__device__ __forceinline__ void chip_cycle(const SPArgs &a, bool first, int *iter, cg::grid_group &grid, double *sh) {
+template <class Sync>
+__device__ __forceinline__ void chip_cycle(const SPArgs &a, bool first, int *iter, Sync &grid, double *sh) {
   using namespace mgs;
   const int top = a.ls + 1, ng = a.ng, t0 = threadIdx.x, bd = blockDim.x;
   int cur[MG_MAX + 1];
@@ -834,9 +836,10 @@ __device__ __noinline__ void split_out(const SPArgs &a, int cur) {
   });
 }
 
+template <class Sync>
 __global__ void __launch_bounds__(SP_BLOCK, 1) k_pdesolver_split(const __grid_constant__ SPArgs a) {
   using namespace mgs;
-  cg::grid_group grid = cg::this_grid();
+  Sync grid;
   __shared__ double sh[64];
   const int ng = a.ng, ls = a.ls, down = ls < ng ? ls : ng - 1;   // down: the last grid level restricted from
   unsigned curs = 0;   // bit l: the current red buffer of grid level l
@@ -1004,10 +1007,11 @@ int launch_split(const int n[3], const double h[3], double *u, const double *b, 
   const int blocks = ctx().sms;
   A.partial = (double *)scratch("mgs_partial", sizeof(double) * 2 * blocks);
   if (!A.partial) return LEPIC_ERR_CUDA;
-  LEPIC_CUDA(cudaFuncSetAttribute(k_pdesolver_split, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csm));
   void *args[] = {&A};
   int tm = timer_start("pdesolver_f64", s);
-  LEPIC_CUDA(cudaLaunchCooperativeKernel((void *)k_pdesolver_split, dim3(blocks), dim3(SP_BLOCK), args, csm, s));
+  LEPIC_CUDA(mgs::launch_solve((const void *)k_pdesolver_split<mgs::GridSync>,
+                               (const void *)k_pdesolver_split<mgs::ClusterSync>, args, A.L[1].len, SP_SMALL, SP_BLOCK,
+                               csm, blocks, s));
   timer_stop(tm, s);
   launched = true;
   return LEPIC_OK;

@@ -29,13 +29,9 @@
 // refinement at 128^3): 128^3 warm 1.53 -> 0.69 ms (4 refinements), 256^3 with
 // electrodes cold 40 -> 16.2 ms (18), 48x80x112 warm 0.72 -> 0.40 ms, 32^3
 // 0.38 -> 0.25 ms.
-#include <cooperative_groups.h>
-
 #include <cstring>
 
 #include "mgsplit.cuh"
-
-namespace cg = cooperative_groups;
 
 namespace lepic {
 
@@ -54,6 +50,7 @@ using Lev = mgs::Lev<float>;
 constexpr int XM_MAX = 13;      // multigrid levels
 constexpr int XM_BLOCK = 512;
 constexpr int XV = 4;           // elements per 16-byte load
+constexpr long long XM_SMALL = 60000;  // elements per colour one cluster solves faster than the grid
 constexpr size_t XM_CHIP = 227000;   // shared memory of the levels on chip
 
 struct XArgs {
@@ -86,8 +83,8 @@ template <bool GRID>
 __device__ __forceinline__ Team team() {
   return GRID ? mgs::grid_team() : mgs::block_team();
 }
-template <bool GRID>
-__device__ __forceinline__ void barrier(cg::grid_group &grid) {
+template <bool GRID, class Sync>
+__device__ __forceinline__ void barrier(Sync &grid) {
   if (GRID)
     grid.sync();
   else
@@ -103,7 +100,8 @@ __device__ __forceinline__ double wsum(double v) {
 // deterministic grid-wide sum of one value per thread, ending at a grid
 // barrier.  The block partials alternate between two halves of a.partial
 // (parity), so one barrier suffices: a half is rewritten two sums later.
-__device__ __forceinline__ double grid_sum(const XArgs &a, double v, int parity, cg::grid_group &grid, double *sh) {
+template <class Sync>
+__device__ __forceinline__ double grid_sum(const XArgs &a, double v, int parity, Sync &grid, double *sh) {
   double *part = a.partial + (parity & 1) * gridDim.x;
   const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
   v = wsum(v);
@@ -207,9 +205,9 @@ __device__ __noinline__ void split_out(const XArgs &a) {
 // nu sweeps of a level.  started: the first red phase is done and black is 0
 // (not written yet); rf: the last black phase also writes the black residual;
 // addu: the last sweep adds its values to u.
-template <bool GRID>
+template <bool GRID, class Sync>
 __device__ __forceinline__ void sweeps(const XArgs &a, const Lev &L, int nu, bool started, bool rf, bool addu,
-                                       cg::grid_group &grid) {
+                                       Sync &grid) {
   using namespace mgs;
   const Team w = team<GRID>();
   const float om = a.omega;
@@ -243,8 +241,8 @@ __device__ __forceinline__ void sweeps(const XArgs &a, const Lev &L, int nu, boo
 
 // the residual of level l (its black half already written when it has been
 // swept) weighted onto level l + 1, whose first red phase is done with it
-template <bool GRID>
-__device__ __forceinline__ void restrict_level(const XArgs &a, int l, bool swept, bool masks, cg::grid_group &grid) {
+template <bool GRID, class Sync>
+__device__ __forceinline__ void restrict_level(const XArgs &a, int l, bool swept, bool masks, Sync &grid) {
   using namespace mgs;
   const Team w = team<GRID>();
   const Lev &F = level_of<GRID>(a, l), &C = level_of<GRID>(a, l + 1);
@@ -258,15 +256,16 @@ __device__ __forceinline__ void restrict_level(const XArgs &a, int l, bool swept
 }
 
 // the sweeps of level l on the way down (or the coarsest level's)
-template <bool GRID>
-__device__ __forceinline__ void down_sweeps(const XArgs &a, int l, bool started, cg::grid_group &grid) {
+template <bool GRID, class Sync>
+__device__ __forceinline__ void down_sweeps(const XArgs &a, int l, bool started, Sync &grid) {
   const bool coarsest = l == a.ng;
   const int nu = coarsest ? a.coarse_sweeps : (l == 1 ? a.nu_fine_pre : a.nu_pre);
   sweeps<GRID>(a, level_of<GRID>(a, l), nu, started, !coarsest, coarsest && a.ng == 1, grid);
 }
 
 // the part of a V-cycle on the levels on chip, by block 0
-__device__ __forceinline__ void chip_cycle(const XArgs &a, bool first, cg::grid_group &grid) {
+template <class Sync>
+__device__ __forceinline__ void chip_cycle(const XArgs &a, bool first, Sync &grid) {
   using namespace mgs;
   const int top = a.ls + 1, ng = a.ng, t0 = threadIdx.x, bd = blockDim.x;
   const Lev &X = level_of<true>(a, top), &T = level_of<false>(a, top);
@@ -319,8 +318,9 @@ __device__ __noinline__ void add_u(const XArgs &a) {
   }
 }
 
+template <class Sync>
 __global__ void __launch_bounds__(XM_BLOCK, 1) k_refine_mixed(const __grid_constant__ XArgs a) {
-  cg::grid_group grid = cg::this_grid();
+  Sync grid;
   __shared__ double sh[32];
   const int ng = a.ng, ls = a.ls, down = ls < ng ? ls : ng - 1;   // down: the last grid level restricted from
   {
@@ -506,7 +506,6 @@ int launch_pdesolver_mixed(const Dims &d, const double h[3], double *u, const do
     }
   }
   A.alpha = fabs((double)((n[0] + 1) * (n[1] + 1) * (n[2] + 1)) * A.ac) * 1.0;
-  LEPIC_CUDA(cudaFuncSetAttribute(k_refine_mixed, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csm));
   const int blocks = c.sms;
   A.partial = (double *)scratch("xm_partial", sizeof(double) * 2 * blocks);
   A.out_i = (int *)scratch("xm_out_i", sizeof(int) * 4);
@@ -514,7 +513,9 @@ int launch_pdesolver_mixed(const Dims &d, const double h[3], double *u, const do
   if (!A.partial || !A.out_i || !A.out_d) return LEPIC_ERR_CUDA;
   void *args[] = {&A};
   int tm = timer_start("pdesolver_mixed", s);
-  LEPIC_CUDA(cudaLaunchCooperativeKernel((void *)k_refine_mixed, dim3(blocks), dim3(XM_BLOCK), args, csm, s));
+  LEPIC_CUDA(mgs::launch_solve((const void *)k_refine_mixed<mgs::GridSync>,
+                               (const void *)k_refine_mixed<mgs::ClusterSync>, args, A.L[1].len, XM_SMALL, XM_BLOCK,
+                               csm, blocks, s));
   timer_stop(tm, s);
   if (!iters && !res_out) {
     // no wait: the solve's status goes to the device error word
