@@ -61,6 +61,29 @@ void *scratch(const char *name, size_t bytes) {
   return b.p;
 }
 
+namespace {
+struct ResultBlock {
+  double *p = nullptr;
+  bool tried = false;
+  ~ResultBlock() {
+    if (p) cudaFreeHost(p);
+  }
+};
+}  // namespace
+
+double *result_block() {
+  static thread_local ResultBlock b;
+  if (!b.tried) {
+    b.tried = true;
+    if (cudaHostAlloc((void **)&b.p, RESULT_WORDS * sizeof(double), cudaHostAllocPortable | cudaHostAllocMapped) !=
+        cudaSuccess) {
+      b.p = nullptr;
+      cudaGetLastError();
+    }
+  }
+  return b.p;
+}
+
 // Synchronise the stream, read and clear the device error word.
 int check_err(cudaStream_t s) {
   Ctx &c = ctx();

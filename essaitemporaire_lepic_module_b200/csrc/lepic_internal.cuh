@@ -45,6 +45,11 @@ struct Ctx {
 Ctx &ctx();                                     // context of the current device
 void *scratch(const char *name, size_t bytes);  // cached device buffer (grows)
 int check_err(cudaStream_t s);                  // sync, read + clear device error word
+// The calling thread's block of pinned host memory for the few results of a
+// kernel that it launches and waits for (the kernel writes them there, which
+// saves two staged copies of about 8 us each); nullptr when there is none.
+constexpr int RESULT_WORDS = 8;
+double *result_block();
 int timer_start(const char *name, cudaStream_t s);  // -1 when timing is off
 void timer_stop(int id, cudaStream_t s);
 int cuda_status(cudaError_t e, const char *what);

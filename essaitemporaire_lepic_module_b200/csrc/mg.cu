@@ -600,6 +600,7 @@ struct SPArgs {
   double *partial;            // [2][gridDim.x]
   int *out_i;
   double *out_d;
+  double *host;               // pinned host memory for k, status, ktot, res (or null)
 };
 
 extern __shared__ __align__(16) unsigned char sp_smem[];
@@ -917,6 +918,12 @@ __global__ void __launch_bounds__(SP_BLOCK, 1) k_pdesolver_split(const __grid_co
     a.out_i[1] = status;
     a.out_d[0] = ktot;
     a.out_d[1] = r;
+    if (a.host) {
+      a.host[0] = k;
+      a.host[1] = status;
+      a.host[2] = ktot;
+      a.host[3] = r;
+    }
   }
 }
 
@@ -938,8 +945,8 @@ int solve_results(const int *out_i, const double *out_d, int *k_out, double *kto
 // does not apply (a level with too many nodes for its 32-bit element numbers,
 // coefficients out of div_by's range): the caller takes the general kernel.
 int launch_split(const int n[3], const double h[3], double *u, const double *b, const int *bcnd, int ncycl,
-                 double eps, double omega, int ng, double eps0, int *out_i, double *out_d, cudaStream_t s,
-                 bool &launched) {
+                 double eps, double omega, int ng, double eps0, int *out_i, double *out_d, double *host,
+                 cudaStream_t s, bool &launched) {
   using Lev = mgs::Lev<double>;
   launched = false;
   if (Lev::elements(n[0], n[1], n[2]) >= 1200000000LL) return LEPIC_OK;
@@ -954,6 +961,7 @@ int launch_split(const int n[3], const double h[3], double *u, const double *b, 
   A.bc = bcnd;
   A.out_i = out_i;
   A.out_d = out_d;
+  A.host = host;
   for (int l = 1; l <= ng; ++l) {
     Lev &L = A.L[l];
     L.shape(n[0] >> (l - 1), n[1] >> (l - 1), n[2] >> (l - 1));
@@ -1032,8 +1040,17 @@ int launch_pdesolver(const Dims &d, const double h[3], double *u, const double *
   double *out_d = (double *)scratch("mg_out_d", sizeof(double) * 2);
   if (!out_i || !out_d) return LEPIC_ERR_CUDA;
   bool launched = false;
+  double *host = gen ? nullptr : result_block();
   if (!gen)
-    if (int rc = launch_split(n, h, u, b, bcnd, ncycl, eps, omega, ng, eps0, out_i, out_d, s, launched)) return rc;
+    if (int rc = launch_split(n, h, u, b, bcnd, ncycl, eps, omega, ng, eps0, out_i, out_d, host, s, launched))
+      return rc;
+  if (launched && host) {
+    LEPIC_CUDA(cudaStreamSynchronize(s));
+    if (k_out) *k_out = (int)host[0];
+    if (ktot_out) *ktot_out = host[2];
+    if (res_out) *res_out = host[3];
+    return (int)host[1];
+  }
   if (launched) return solve_results(out_i, out_d, k_out, ktot_out, res_out, s);
   MGArgs A;
   memset(&A, 0, sizeof(A));

@@ -69,6 +69,7 @@ struct XArgs {
   double *partial;            // [2][gridDim.x]
   int *out_i;      // [0] refinement iterations, [1] status
   double *out_d;   // [0] res/alpha, [1] first res/alpha
+  double *host;    // pinned host memory for refinements, status, res/alpha (or null)
 };
 
 extern __shared__ __align__(16) unsigned char xm_smem[];
@@ -407,6 +408,11 @@ __global__ void __launch_bounds__(XM_BLOCK, 1) k_refine_mixed(const __grid_const
     a.out_i[1] = status;
     a.out_d[0] = res;
     a.out_d[1] = res0;
+    if (a.host) {
+      a.host[0] = it;
+      a.host[1] = status;
+      a.host[2] = res;
+    }
   }
 }
 
@@ -511,17 +517,25 @@ int launch_pdesolver_mixed(const Dims &d, const double h[3], double *u, const do
   A.out_i = (int *)scratch("xm_out_i", sizeof(int) * 4);
   A.out_d = (double *)scratch("xm_out_d", sizeof(double) * 2);
   if (!A.partial || !A.out_i || !A.out_d) return LEPIC_ERR_CUDA;
+  const bool wait = iters || res_out;
+  A.host = wait ? result_block() : nullptr;
   void *args[] = {&A};
   int tm = timer_start("pdesolver_mixed", s);
   LEPIC_CUDA(mgs::launch_solve((const void *)k_refine_mixed<mgs::GridSync>,
                                (const void *)k_refine_mixed<mgs::ClusterSync>, args, A.L[1].len, XM_SMALL, XM_BLOCK,
                                csm, blocks, s));
   timer_stop(tm, s);
-  if (!iters && !res_out) {
+  if (!wait) {
     // no wait: the solve's status goes to the device error word
     k_solve_status<<<1, 1, 0, s>>>(A.out_i, ctx().d_err);
     LEPIC_CUDA(cudaGetLastError());
     return LEPIC_OK;
+  }
+  if (A.host) {
+    LEPIC_CUDA(cudaStreamSynchronize(s));
+    if (iters) *iters = (int)A.host[0];
+    if (res_out) *res_out = A.host[2];
+    return (int)A.host[1];
   }
   int hi[4];
   double hd[2];
