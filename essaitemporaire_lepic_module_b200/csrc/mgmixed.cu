@@ -48,7 +48,11 @@ using mgs::Team;
 using Lev = mgs::Lev<float>;
 
 constexpr int XM_MAX = 13;      // multigrid levels
-constexpr int XM_BLOCK = 512;
+// threads per block: twice as many, at half the registers, on grids whose
+// finest level moves through HBM (a solve at 256^3: 13.9 -> 12.7 ms; at 192^3
+// and 176^3 the same; at 160^3 10.4 -> 11.3 ms, at 128^3 617 -> 714 us)
+constexpr int XM_BLOCK = 512, XM_BLOCK_LARGE = 1024;
+constexpr long long XM_LARGE = 3000000;   // elements per colour from which it takes those
 constexpr int XV = 4;           // elements per 16-byte load
 constexpr long long XM_SMALL = 60000;  // elements per colour one cluster solves faster than the grid
 constexpr size_t XM_CHIP = 227000;   // shared memory of the levels on chip
@@ -319,8 +323,8 @@ __device__ __noinline__ void add_u(const XArgs &a) {
   }
 }
 
-template <class Sync>
-__global__ void __launch_bounds__(XM_BLOCK, 1) k_refine_mixed(const __grid_constant__ XArgs a) {
+template <class Sync, int BLOCK>
+__global__ void __launch_bounds__(BLOCK, 1) k_refine_mixed(const __grid_constant__ XArgs a) {
   Sync grid;
   __shared__ double sh[32];
   const int ng = a.ng, ls = a.ls, down = ls < ng ? ls : ng - 1;   // down: the last grid level restricted from
@@ -521,9 +525,11 @@ int launch_pdesolver_mixed(const Dims &d, const double h[3], double *u, const do
   A.host = wait ? result_block() : nullptr;
   void *args[] = {&A};
   int tm = timer_start("pdesolver_mixed", s);
-  LEPIC_CUDA(mgs::launch_solve((const void *)k_refine_mixed<mgs::GridSync>,
-                               (const void *)k_refine_mixed<mgs::ClusterSync>, args, A.L[1].len, XM_SMALL, XM_BLOCK,
-                               csm, blocks, s));
+  const bool large = A.L[1].len >= XM_LARGE;
+  LEPIC_CUDA(mgs::launch_solve(large ? (const void *)k_refine_mixed<mgs::GridSync, XM_BLOCK_LARGE>
+                                     : (const void *)k_refine_mixed<mgs::GridSync, XM_BLOCK>,
+                               (const void *)k_refine_mixed<mgs::ClusterSync, XM_BLOCK>, args, A.L[1].len, XM_SMALL,
+                               large ? XM_BLOCK_LARGE : XM_BLOCK, csm, blocks, s));
   timer_stop(tm, s);
   if (!wait) {
     // no wait: the solve's status goes to the device error word
