@@ -38,6 +38,7 @@ constexpr int MAX_LABEL = 16;
 struct WinConst {
   double h0, h1, h2, dt, k1, kk, Bx, By, Bz, kdep, q, mass;
   double r0, r1, r2;  // 1 / h, rounded
+  double d0, d1, d2;  // dt / h
   double dkk;       // d kk / d Bz
   double Nm;        // macroparticle weight
   int boris;
@@ -549,6 +550,9 @@ WinConst win_const(const lepic_grid_t &g, const lepic_phys_t &P, int ptype) {
   c.r1 = 1.0 / c.h1;
   c.r2 = 1.0 / c.h2;
   c.dt = P.dt;
+  c.d0 = c.dt / c.h0;
+  c.d1 = c.dt / c.h1;
+  c.d2 = c.dt / c.h2;
   c.k1 = P.dt * P.charge[p] / (2.0 * P.mass[p]);
   c.Bx = P.Bconst[0];
   c.By = P.Bconst[1];
@@ -871,40 +875,62 @@ __device__ void flush_qbox(const Dims &d, unsigned *box, int bx, int by, int bz,
 }
 static_assert(qsum_window_ok(WFLUSH), "node sums of a flush window are read back modulo 2^32");
 
-// the FP32 window's deposit, one block per tile: the integer weights of the
-// mixed step (2^20 units per particle), summed exactly in a 32-bit node box
-__global__ void __launch_bounds__(AB) k_cw_deposit_tiles(Dims d, WinConst c, WinS<float> S, const int *__restrict__ count,
-                                                         WinTiles T, int step, const double *__restrict__ kq,
-                                                         double *__restrict__ np) {
-  __shared__ unsigned s_box[WBN];
-  int bx, by, bz;
-  tile_box(T, blockIdx.x, bx, by, bz);
-  for (int e = threadIdx.x; e < WBN; e += AB) s_box[e] = 0u;
-  __syncthreads();
+// the FP32 window's deposit: the integer weights of the mixed step (2^20 units
+// per particle), summed exactly in a 32-bit node box per block.  As in the
+// step loop's deposit, a window of WFLUSH slots (history word, cell, offsets)
+// is staged by cp.async while the box of the window before is flushed, and
+// lane l works through the l-th WFLUSH / 32 slots of it, so that the lanes of
+// a warp add to the words of different cells (neighbouring slots share their
+// cell: summing them over the warp first cost three times the weights).
+constexpr int WDL = WFLUSH / 32;            // slots per lane
+static_assert(WDL % 32 == 0 && WFLUSH % AB == 0 && (AB / 32) * (WFLUSH / AB) == WDL,
+              "a window is each lane's part, dealt to the warps");
+constexpr int CW_DEP_SMEM = 20 * WFLUSH + 4 * WBN;
+__global__ void __launch_bounds__(AB, 4) k_cw_deposit_tiles(Dims d, WinConst c, WinS<float> S,
+                                                            const int *__restrict__ count, WinTiles T, int step,
+                                                            const double *__restrict__ kq, double *__restrict__ np) {
+  extern __shared__ __align__(16) unsigned char s_dep[];
+  int *s_bl = reinterpret_cast<int *>(s_dep), *s_cell = s_bl + WFLUSH;
+  float *s_f = reinterpret_cast<float *>(s_cell + WFLUSH);      // [3][WFLUSH]
+  unsigned *s_box = reinterpret_cast<unsigned *>(s_f + 3 * WFLUSH);
   const long long N = *count;
   const long long lo = T.off[blockIdx.x];
   long long hi = T.off[blockIdx.x + 1];
   if (hi > N) hi = N;
-  int chunks = 0;
-  for (long long base = lo; base < hi; base += AB) {
-    // every lane takes part in the run sums (base is uniform over the block)
-    const long long i = base + threadIdx.x;
-    int ix = 0, iy = 0, iz = 0;
-    int w[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    long long key = -1;
-    float wf[8];
-    if (i < hi && cw_dep_one<float>(S, i, step, ix, iy, iz, wf)) {
-      key = d.g(ix, iy, iz);
-      qweights(S.p[i], S.p[S.cap + i], S.p[2 * S.cap + i], w);
+  int bx, by, bz;
+  tile_box(T, blockIdx.x, bx, by, bz);
+  auto fetch = [&](long long base) {
+    for (int q = threadIdx.x; q < WFLUSH; q += AB) {
+      const long long i = base + q;
+      if (i >= hi) break;
+      cp_async4(s_bl + q, S.bl + i);
+      cp_async4(s_cell + q, S.cell + i);
+#pragma unroll
+      for (int a = 0; a < 3; ++a) cp_async4(s_f + a * WFLUSH + q, S.p + a * S.cap + i);
     }
-    // the lanes of one cell (consecutive in the sort's order) are summed
-    // first, so a cell's particles do not contend for the same shared words
-    if (warp_run_sum<8, int>(key, w)) {
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  fetch(lo);
+  for (int e = threadIdx.x; e < WBN; e += AB) s_box[e] = 0u;
+  const int lane = threadIdx.x & 31, part = (threadIdx.x >> 5) * (WFLUSH / AB);
+  for (long long base = lo; base < hi; base += WFLUSH) {
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+#pragma unroll 2
+    for (int k = 0; k < WFLUSH / AB; ++k) {
+      const int s = lane * WDL + ((part + k + lane) & (WDL - 1));
+      if (base + s >= hi) continue;
+      const int b = s_bl[s];
+      if (!(born_of(b) < step && lost_of(b) >= step)) continue;
+      int ix, iy, iz, w[8];
+      unpack_cell(s_cell[s], ix, iy, iz);
+      qweights(s_f[s], s_f[WFLUSH + s], s_f[2 * WFLUSH + s], w);
       const int b0 = box_base(ix, iy, iz, bx, by, bz);
       if (b0 >= 0) {
 #pragma unroll
         for (int q = 0; q < 8; ++q) atomicAdd(&s_box[b0 + box_off(q)], (unsigned)w[q]);
       } else {
+        const long long key = d.g(ix, iy, iz);
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
           const long long g = key + ox(q) + d.N1 * (oy(q) + d.N2 * (long long)oz(q));
@@ -912,15 +938,10 @@ __global__ void __launch_bounds__(AB) k_cw_deposit_tiles(Dims d, WinConst c, Win
         }
       }
     }
-    if (++chunks == WFLUSH / AB && base + AB < hi) {
-      chunks = 0;
-      __syncthreads();
-      flush_qbox(d, s_box, bx, by, bz, kq, c.kdep, np);
-      __syncthreads();
-    }
+    __syncthreads();
+    if (base + WFLUSH < hi) fetch(base + WFLUSH);
+    flush_qbox(d, s_box, bx, by, bz, kq, c.kdep, np);
   }
-  __syncthreads();
-  flush_qbox(d, s_box, bx, by, bz, kq, c.kdep, np);
 }
 
 // E gathers of a cell's 8 nodes in the order of gather_E: from the FP32 /
@@ -1005,9 +1026,9 @@ __device__ __forceinline__ void cw_push_one(const Dims &d, const WinConst &c, co
   R Ex, Ey, Ez;
   gather(ix, iy, iz, w, Ex, Ey, Ez);
   boris<R>(c, Ex, Ey, Ez, vx, vy, vz);
-  const int ax = ix + move_offset<R>(fx, vx * (R)(c.dt / c.h0));
-  const int ay = iy + move_offset<R>(fy, vy * (R)(c.dt / c.h1));
-  const int az = iz + move_offset<R>(fz, vz * (R)(c.dt / c.h2));
+  const int ax = ix + move_offset<R>(fx, vx * (R)c.d0);
+  const int ay = iy + move_offset<R>(fy, vy * (R)c.d1);
+  const int az = iz + move_offset<R>(fz, vz * (R)c.d2);
   const int cx = ax < 0 ? 0 : (ax > d.n1 + 1 ? d.n1 + 1 : ax);
   const int cy = ay < 0 ? 0 : (ay > d.n2 + 1 ? d.n2 + 1 : ay);
   const int cz = az < 0 ? 0 : (az > d.n3 + 1 ? d.n3 + 1 : az);
@@ -1073,36 +1094,34 @@ __global__ void __launch_bounds__(AB, 3) k_cw_push_tiles(Dims d, WinConst c, con
 }
 
 // the push of step `step` undone for the particles it kept: x^n from
-// x^{n+1} and v^{n+1/2}, then v+ by the inverse rotation with E^n at x^n
-// on a state in registers: true when the push of `step` was undone (st
-// updated in place)
+// x^{n+1} and v^{n+1/2} (cw_move_back), then v+ by the inverse rotation with
+// E^n at x^n.  On a state in registers: true when the push of `step` was
+// undone (st updated in place).
+template <class R>
+__device__ __forceinline__ void cw_move_back(const Dims &d, const WinConst &c, PSt<R> &st) {
+  int ix, iy, iz;
+  unpack_cell(st.cell, ix, iy, iz);
+  ix += move_offset<R>(st.f[0], -st.v[0] * (R)c.d0);
+  iy += move_offset<R>(st.f[1], -st.v[1] * (R)c.d1);
+  iz += move_offset<R>(st.f[2], -st.v[2] * (R)c.d2);
+  ix = ix < 1 ? 1 : (ix > d.n1 ? d.n1 : ix);
+  iy = iy < 1 ? 1 : (iy > d.n2 ? d.n2 : iy);
+  iz = iz < 1 ? 1 : (iz > d.n3 ? d.n3 : iz);
+  st.cell = pack_cell(ix, iy, iz);
+}
 template <class R, class G>
 __device__ __forceinline__ bool cw_reverse_core(const Dims &d, const WinConst &c, PSt<R> &st, int step,
                                                 const G &gather) {
   const int b = st.b;
   if (!(born_of(b) <= step && lost_of(b) > step)) return false;
+  cw_move_back<R>(d, c, st);
   int ix, iy, iz;
   unpack_cell(st.cell, ix, iy, iz);
-  R fx = st.f[0], fy = st.f[1], fz = st.f[2];
-  R vx = st.v[0], vy = st.v[1], vz = st.v[2];
-  ix += move_offset<R>(fx, -vx * (R)(c.dt / c.h0));
-  iy += move_offset<R>(fy, -vy * (R)(c.dt / c.h1));
-  iz += move_offset<R>(fz, -vz * (R)(c.dt / c.h2));
-  ix = ix < 1 ? 1 : (ix > d.n1 ? d.n1 : ix);
-  iy = iy < 1 ? 1 : (iy > d.n2 ? d.n2 : iy);
-  iz = iz < 1 ? 1 : (iz > d.n3 ? d.n3 : iz);
   R w[8];
-  weights8<R>(fx, fy, fz, w);
+  weights8<R>(st.f[0], st.f[1], st.f[2], w);
   R Ex, Ey, Ez;
   gather(ix, iy, iz, w, Ex, Ey, Ez);
-  boris_inverse<R>(c, Ex, Ey, Ez, vx, vy, vz);
-  st.cell = pack_cell(ix, iy, iz);
-  st.f[0] = fx;
-  st.f[1] = fy;
-  st.f[2] = fz;
-  st.v[0] = vx;
-  st.v[1] = vy;
-  st.v[2] = vz;
+  boris_inverse<R>(c, Ex, Ey, Ez, st.v[0], st.v[1], st.v[2]);
   return true;
 }
 
@@ -1167,15 +1186,16 @@ __global__ void __launch_bounds__(AB, 3) k_cw_reverse_tiles(Dims d, WinConst c, 
 // On a state and adjoint held in registers: st the particle at (x^n, v+),
 // lam in: (dJ/dx^{n+1}, dJ/dv^{n+1/2}), out: the push's part of dJ/dx^n and
 // dJ/dv+ (a particle lost at this step starts from zero, or from wflux).
+// undo: st comes at (x^n, v^{n+1/2}) and leaves at (x^n, v+), the push's
+// rotation undone with the same gathered E.
 template <class R, class N>
-__device__ __forceinline__ bool cw_adj_push_core(const WinConst &c, const N &nodes, const PSt<R> &st, int step,
+__device__ __forceinline__ bool cw_adj_push_core(const WinConst &c, const N &nodes, PSt<R> &st, int step, bool undo,
                                                  double wflux, R (&lam)[6], int &ix, int &iy, int &iz,
                                                  R (&sc)[24], double &gB) {
   const int b = st.b;
   if (!(born_of(b) <= step && lost_of(b) >= step)) return false;
   unpack_cell(st.cell, ix, iy, iz);
   const R fx = st.f[0], fy = st.f[1], fz = st.f[2];
-  const R vx = st.v[0], vy = st.v[1], vz = st.v[2];
   R w[8];
   weights8<R>(fx, fy, fz, w);
   // E at the cell's 8 nodes, read once for the gather and its weight gradient
@@ -1188,6 +1208,8 @@ __device__ __forceinline__ bool cw_adj_push_core(const WinConst &c, const N &nod
     Ey += w[q] * en[q][1];
     Ez += w[q] * en[q][2];
   }
+  if (undo) boris_inverse<R>(c, Ex, Ey, Ez, st.v[0], st.v[1], st.v[2]);
+  const R vx = st.v[0], vy = st.v[1], vz = st.v[2];
   R lx, ly, lz, lvx, lvy, lvz;
   if (lost_of(b) == step) {
     lx = ly = lz = R(0);
@@ -1247,7 +1269,7 @@ __device__ __forceinline__ bool cw_adj_push_core(const WinConst &c, const N &nod
   }
   // gather^T and the weight gradient of the gather into lx
   const R px = R(1) - fx, py = R(1) - fy, pz = R(1) - fz;
-  const R hx = (R)(1.0 / c.h0), hy = (R)(1.0 / c.h1), hz = (R)(1.0 / c.h2);
+  const R hx = (R)c.r0, hy = (R)c.r1, hz = (R)c.r2;
 #pragma unroll
   for (int q = 0; q < 8; ++q) {
     sc[3 * q + 0] = w[q] * lEx;
@@ -1281,7 +1303,7 @@ __device__ __forceinline__ bool cw_adj_push_one(const WinConst &c, const N &node
   R lam[6];
 #pragma unroll
   for (int a = 0; a < 6; ++a) lam[a] = S.lam[a * cap + i];
-  cw_adj_push_core<R>(c, nodes, st, step, wflux, lam, ix, iy, iz, sc, gB);
+  cw_adj_push_core<R>(c, nodes, st, step, false, wflux, lam, ix, iy, iz, sc, gB);
 #pragma unroll
   for (int a = 0; a < 6; ++a) S.lam[a * cap + i] = lam[a];
   return true;
@@ -1427,8 +1449,7 @@ __device__ __forceinline__ void cw_adj_dep_core(const WinConst &c, double fx, do
   for (int q = 0; q < 8; ++q) {
     const double s = m(q);
     const double ax = ox(q) ? 1.0 - px : px, ay = oy(q) ? 1.0 - py : py, az = oz(q) ? 1.0 - pz : pz;
-    const double sx = ox(q) ? 1.0 / c.h0 : -1.0 / c.h0, sy = oy(q) ? 1.0 / c.h1 : -1.0 / c.h1,
-                 sz = oz(q) ? 1.0 / c.h2 : -1.0 / c.h2;
+    const double sx = ox(q) ? c.r0 : -c.r0, sy = oy(q) ? c.r1 : -c.r1, sz = oz(q) ? c.r2 : -c.r2;
     lx += sx * ay * az * s;
     ly += ax * sy * az * s;
     lz += ax * ay * sz * s;
@@ -1447,8 +1468,7 @@ __device__ __forceinline__ void cw_adj_dep_one(const WinConst &c, const WinS<R> 
   for (int q = 0; q < 8; ++q) {
     const double s = m(q);
     const double ax = ox(q) ? 1.0 - px : px, ay = oy(q) ? 1.0 - py : py, az = oz(q) ? 1.0 - pz : pz;
-    const double sx = ox(q) ? 1.0 / c.h0 : -1.0 / c.h0, sy = oy(q) ? 1.0 / c.h1 : -1.0 / c.h1,
-                 sz = oz(q) ? 1.0 / c.h2 : -1.0 / c.h2;
+    const double sx = ox(q) ? c.r0 : -c.r0, sy = oy(q) ? c.r1 : -c.r1, sz = oz(q) ? c.r2 : -c.r2;
     lx += sx * ay * az * s;
     ly += ax * sy * az * s;
     lz += ax * ay * sz * s;
@@ -1583,7 +1603,6 @@ __global__ void __launch_bounds__(AB, 2) k_cw_back_tiles(Dims d, WinConst c, con
   }
   for (int e = threadIdx.x; e < 3 * WBN; e += AB) s_box[e] = 0.f;
   __syncthreads();
-  const ETile G{d, E, s_E, bx, by, bz};
   const ENodesTile nodes{d, E, s_E, bx, by, bz};
   double gB = 0.0;
   int chunks = 0;
@@ -1634,8 +1653,13 @@ __global__ void __launch_bounds__(AB, 2) k_cw_back_tiles(Dims d, WinConst c, con
         lam[2] += (float)lz;
         lam_changed = true;
       }
-      if (cw_reverse_core<float>(d, c, st, step, G)) pst_store<float>(S, i, st);
-      if (cw_adj_push_core<float>(c, nodes, st, step, wflux, lam, ix, iy, iz, r, gB)) {
+      // the push of `step` undone, E at x^step read once for that and for the
+      // adjoint of the push
+      const bool kept = born_of(st.b) <= step && lost_of(st.b) > step;
+      if (kept) cw_move_back<float>(d, c, st);
+      const bool pushed = cw_adj_push_core<float>(c, nodes, st, step, kept, wflux, lam, ix, iy, iz, r, gB);
+      if (kept) pst_store<float>(S, i, st);
+      if (pushed) {
         key = d.g(ix, iy, iz);
         b0 = box_base(ix, iy, iz, bx, by, bz);
         lam_changed = true;
@@ -1899,8 +1923,10 @@ int lepic_dev_cw_deposit(const lepic_grid_t *g, const lepic_win_species_t *ws, i
     long long first = 0;
     if (ws->tile_off) {
       const lepic::WinTiles T = lepic::win_tiles(*g, *ws);
-      lepic::k_cw_deposit_tiles<<<LEPIC_TILES(g->n), lepic::AB, 0, s>>>(d, c, lepic::win_view<float>(*ws), ws->count,
-                                                                         T, step, g->kq, np);
+      LEPIC_CUDA(cudaFuncSetAttribute(lepic::k_cw_deposit_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      lepic::CW_DEP_SMEM));
+      lepic::k_cw_deposit_tiles<<<LEPIC_TILES(g->n), lepic::AB, lepic::CW_DEP_SMEM, s>>>(
+          d, c, lepic::win_view<float>(*ws), ws->count, T, step, g->kq, np);
       first = ws->tile_end;
     }
     lepic::k_cw_deposit<float><<<lepic::grid_for(ws->cap - first, lepic::AB), lepic::AB, 0, s>>>(
