@@ -525,20 +525,26 @@ __device__ __forceinline__ void push_quad(const Dims &d, const MixedConst &c, co
         for (int a = 0; a < 6; ++a) p[a * cap + i0 + k] = (&P[a].x)[k];
       }
   }
-  // holes: flag 2 and a warp-aggregated append to the hole list
+  // holes: flag 2 and an append to the hole list, one atomic for the warp's
+  // four quads of lanes together (its round trip stalls the warp)
   const int lane = threadIdx.x & 31;
   if (__any_sync(full, hole[0] | hole[1] | hole[2] | hole[3])) {
+    unsigned hm[4];
+    int before[4], total = 0;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      if (hole[k]) flag[i0 + k] = 2;
-      const unsigned hm = __ballot_sync(full, hole[k]);
-      if (hm) {
-        const int leader = __ffs(hm) - 1;
-        int base = 0;
-        if (lane == leader) base = atomicAdd(nholes, __popc(hm));
-        base = __shfl_sync(full, base, leader);
-        if (hole[k]) holes[base + __popc(hm & lmask_lt())] = (int)(i0 + k);
-      }
+      hm[k] = __ballot_sync(full, hole[k]);
+      before[k] = total;
+      total += __popc(hm[k]);
+    }
+    int base = 0;
+    if (lane == 0) base = atomicAdd(nholes, total);
+    base = __shfl_sync(full, base, 0);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (!hole[k]) continue;
+      flag[i0 + k] = 2;
+      holes[base + before[k] + __popc(hm[k] & lmask_lt())] = (int)(i0 + k);
     }
   }
   if (DEP) deposit_quad(d, T, jx, jy, jz, gxs, gys, gzs, c.kdep, kq, np);
