@@ -1,4 +1,5 @@
 // Per-device context: error word, scratch buffers, status helpers.
+#include <atomic>
 #include <cstring>
 #include <map>
 #include <mutex>
@@ -17,6 +18,8 @@ struct Buf {
 };
 std::map<std::pair<int, std::string>, Buf> g_scratch;
 thread_local int g_last_cuda_error = 0;
+constexpr unsigned BARRIERS = 64, BARRIER_WORDS = 32;   // a 128-byte line each
+std::atomic<unsigned> g_barrier{0};
 }  // namespace
 
 int cuda_status(cudaError_t e, const char *what) {
@@ -38,8 +41,17 @@ Ctx &ctx() {
     cudaMemset(c.d_err, 0, 2 * sizeof(int));
     cudaMallocHost(&c.h_err, 2 * sizeof(int));
     c.h_err[0] = c.h_err[1] = 0;
+    if (cudaMalloc(&c.d_barrier, BARRIERS * BARRIER_WORDS * sizeof(unsigned)) == cudaSuccess)
+      cudaMemset(c.d_barrier, 0, BARRIERS * BARRIER_WORDS * sizeof(unsigned));
+    else
+      c.d_barrier = nullptr;
   }
   return c;
+}
+
+unsigned *grid_barrier() {
+  Ctx &c = ctx();
+  return c.d_barrier ? c.d_barrier + (g_barrier++ % BARRIERS) * BARRIER_WORDS : nullptr;
 }
 
 void *scratch(const char *name, size_t bytes) {
@@ -95,6 +107,9 @@ int check_err(cudaStream_t s) {
   if (code) {
     fprintf(stderr, "lepic_gpu: device status %d (detail %d)\n", code, c.h_err[1]);
     cudaMemsetAsync(c.d_err, 0, 2 * sizeof(int), s);
+    // a barrier that was given up has left its word between two states
+    if (code == LEPIC_ERR_TIMEOUT && c.d_barrier)
+      cudaMemsetAsync(c.d_barrier, 0, BARRIERS * BARRIER_WORDS * sizeof(unsigned), s);
     cudaStreamSynchronize(s);
   }
   return code;

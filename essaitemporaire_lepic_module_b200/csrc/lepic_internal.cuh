@@ -40,6 +40,7 @@ struct Ctx {
   int sms = 0;
   int *d_err = nullptr;       // device int[2]
   int *h_err = nullptr;       // pinned host int[2]
+  unsigned *d_barrier = nullptr;   // the words of grid_barrier()
   cudaDeviceProp prop{};
 };
 Ctx &ctx();                                     // context of the current device
@@ -50,6 +51,10 @@ int check_err(cudaStream_t s);                  // sync, read + clear device err
 // saves two staged copies of about 8 us each); nullptr when there is none.
 constexpr int RESULT_WORDS = 8;
 double *result_block();
+// A barrier word for one launch of a kernel over the whole device, in device
+// memory and in the state every launch leaves behind.  They are handed out in
+// turn, so launches that overlap have different ones.
+unsigned *grid_barrier();
 int timer_start(const char *name, cudaStream_t s);  // -1 when timing is off
 void timer_stop(int id, cudaStream_t s);
 int cuda_status(cudaError_t e, const char *what);

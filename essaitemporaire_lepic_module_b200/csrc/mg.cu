@@ -601,6 +601,8 @@ struct SPArgs {
   int *out_i;
   double *out_d;
   double *host;               // pinned host memory for k, status, ktot, res (or null)
+  unsigned *barrier;          // this launch's barrier word, the device error word
+  int *err;
 };
 
 extern __shared__ __align__(16) unsigned char sp_smem[];
@@ -840,7 +842,7 @@ __device__ __noinline__ void split_out(const SPArgs &a, int cur) {
 template <class Sync>
 __global__ void __launch_bounds__(SP_BLOCK, 1) k_pdesolver_split(const __grid_constant__ SPArgs a) {
   using namespace mgs;
-  Sync grid;
+  Sync grid(a.barrier, a.err);
   __shared__ double sh[64];
   const int ng = a.ng, ls = a.ls, down = ls < ng ? ls : ng - 1;   // down: the last grid level restricted from
   unsigned curs = 0;   // bit l: the current red buffer of grid level l
@@ -962,6 +964,9 @@ int launch_split(const int n[3], const double h[3], double *u, const double *b, 
   A.out_i = out_i;
   A.out_d = out_d;
   A.host = host;
+  A.barrier = grid_barrier();
+  A.err = ctx().d_err;
+  if (!A.barrier) return LEPIC_ERR_CUDA;
   for (int l = 1; l <= ng; ++l) {
     Lev &L = A.L[l];
     L.shape(n[0] >> (l - 1), n[1] >> (l - 1), n[2] >> (l - 1));

@@ -74,6 +74,8 @@ struct XArgs {
   int *out_i;      // [0] refinement iterations, [1] status
   double *out_d;   // [0] res/alpha, [1] first res/alpha
   double *host;    // pinned host memory for refinements, status, res/alpha (or null)
+  unsigned *barrier;   // this launch's barrier word, the device error word
+  int *err;
 };
 
 extern __shared__ __align__(16) unsigned char xm_smem[];
@@ -325,7 +327,7 @@ __device__ __noinline__ void add_u(const XArgs &a) {
 
 template <class Sync, int BLOCK>
 __global__ void __launch_bounds__(BLOCK, 1) k_refine_mixed(const __grid_constant__ XArgs a) {
-  Sync grid;
+  Sync grid(a.barrier, a.err);
   __shared__ double sh[32];
   const int ng = a.ng, ls = a.ls, down = ls < ng ? ls : ng - 1;   // down: the last grid level restricted from
   {
@@ -451,6 +453,9 @@ int launch_pdesolver_mixed(const Dims &d, const double h[3], double *u, const do
   A.b = b;
   A.bcnd = bcnd;
   A.eps = eps;
+  A.barrier = grid_barrier();
+  A.err = c.d_err;
+  if (!A.barrier) return LEPIC_ERR_CUDA;
   if (Lev::elements(n[0], n[1], n[2]) >= 1200000000LL) return LEPIC_ERR_UNSUPPORTED;   // 32-bit element numbers
   // shapes and coefficients per level (Src/mg.h)
   for (int l = 1; l <= ng; ++l) {
