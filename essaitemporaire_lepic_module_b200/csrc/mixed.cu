@@ -811,7 +811,13 @@ __global__ void k_tile_offsets(const int *__restrict__ off, int ntiles, int *__r
 
 // The sort's chunks: SC_N consecutive particles per block, counted per key in
 // a shared-memory table (open addressing on the key).
-constexpr int SC_T = 256, SC_U = 4, SC_N = SC_T * SC_U, SC_H = 1024, SC_HBITS = 10;
+// The scatter holds its particles in registers meanwhile and is bound by the
+// latency of its phases: 48 warps per SM with two particles a thread take 3.31
+// ms per 1.25e8 particles at 128^3, 32 warps with four 3.46.  (The histogram
+// has four a thread: 0.60 ms against 0.68.)
+constexpr int SC_T = 512, SC_U = 2, SC_N = SC_T * SC_U, SC_H = 1024, SC_HBITS = 10;
+constexpr int SH_T = 256, SH_U = 4;
+static_assert(SH_T * SH_U == SC_N, "the same chunks");
 constexpr size_t SC_SMEM = sizeof(int) * (4 * SC_H + 2 * SC_N) + sizeof(float) * 6 * SC_N;
 static_assert(SC_H >= SC_N, "the table holds every distinct key of a chunk");
 
@@ -843,7 +849,7 @@ __device__ __forceinline__ void table_add(int key, int *hkey, int *hcnt, int &sl
 // distinct key with a single atomic on that key's cursor, stages the
 // particles in key order and writes them out so that consecutive threads
 // store consecutive slots of a key's range.
-__global__ void __launch_bounds__(SC_T, 4) k_msort_scatter(const int *__restrict__ cell, const float *__restrict__ p,
+__global__ void __launch_bounds__(SC_T, 3) k_msort_scatter(const int *__restrict__ cell, const float *__restrict__ p,
                                                            int *__restrict__ cell_o, float *__restrict__ p_o,
                                                            long long cap, const int *__restrict__ count, int ntx,
                                                            int nty, int *__restrict__ cursor) {
@@ -881,7 +887,7 @@ __global__ void __launch_bounds__(SC_T, 4) k_msort_scatter(const int *__restrict
   }
   __syncthreads();
   {
-    // exclusive scan of the slot counts (four slots per thread), then one
+    // exclusive scan of the slot counts (PER slots per thread), then one
     // range per distinct key from its global cursor
     constexpr int PER = SC_H / SC_T;
     int v[PER];
@@ -930,31 +936,31 @@ __global__ void __launch_bounds__(SC_T, 4) k_msort_scatter(const int *__restrict
 
 // Counts per key of the counting sort: each distinct key of a chunk adds its
 // count to the global histogram once.
-__global__ void __launch_bounds__(SC_T) k_msort_hist(const int *__restrict__ cell, const int *__restrict__ count,
+__global__ void __launch_bounds__(SH_T) k_msort_hist(const int *__restrict__ cell, const int *__restrict__ count,
                                                      int ntx, int nty, int *__restrict__ cnt) {
   __shared__ int hkey[SC_H], hcnt[SC_H];
   const int t = threadIdx.x;
   const long long N = *count;
   const long long c0 = (long long)blockIdx.x * SC_N;
   if (c0 >= N) return;  // uniform over the block
-  for (int q = t; q < SC_H; q += SC_T) {
+  for (int q = t; q < SC_H; q += SH_T) {
     hkey[q] = -1;
     hcnt[q] = 0;
   }
-  int key[SC_U];
+  int key[SH_U];
 #pragma unroll
-  for (int u = 0; u < SC_U; ++u) {
-    const long long idx = c0 + u * SC_T + t;
+  for (int u = 0; u < SH_U; ++u) {
+    const long long idx = c0 + u * SH_T + t;
     key[u] = idx < N ? cell[idx] : -1;
   }
   __syncthreads();
 #pragma unroll
-  for (int u = 0; u < SC_U; ++u) {
+  for (int u = 0; u < SH_U; ++u) {
     int slot, rank;
     table_add(key[u] < 0 ? -1 : tile_key(key[u], ntx, nty), hkey, hcnt, slot, rank);
   }
   __syncthreads();
-  for (int q = t; q < SC_H; q += SC_T)
+  for (int q = t; q < SC_H; q += SH_T)
     if (hcnt[q]) atomicAdd(&cnt[hkey[q]], hcnt[q]);
 }
 
@@ -1251,7 +1257,7 @@ int launch_sort_mixed(const lepic_grid_t &g, lepic_species_mixed_t &sp, int n_hi
   LEPIC_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int) * (size_t)(nkeys + 1), s));
   const int nthreads = n_hint > 0 ? n_hint : sp.cap;
   int t0 = timer_start("sort_hist_mixed", s);
-  k_msort_hist<<<grid_for(nthreads, SC_N), SC_T, 0, s>>>(sp.cell, sp.count, ntx, nty, cnt);
+  k_msort_hist<<<grid_for(nthreads, SC_N), SH_T, 0, s>>>(sp.cell, sp.count, ntx, nty, cnt);
   timer_stop(t0, s);
   int t1 = timer_start("sort_scan_mixed", s);
   int rc = exclusive_scan_i32(cnt, cnt, nkeys + 1, s);
