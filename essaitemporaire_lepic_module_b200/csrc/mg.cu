@@ -683,10 +683,10 @@ __device__ __forceinline__ double smooth(const SPArgs &a, int level, int &cur, b
     if (l == 1 && started) {
       cur ^= 1;   // taken back below: the values stand in the current buffer
     } else if (l == 1) {
-      colour_phase<double, 2, RED, DO_RELAX>(L, L.red[cur], L.red[cur ^ 1], L.black, om, w);
+      colour_phase<double, 2, RED, DO_RELAX, !GRID>(L, L.red[cur], L.red[cur ^ 1], L.black, om, w);
       barrier();
     } else {
-      part += colour_phase<double, 2, RED, DO_RELAX | DO_RES>(L, L.red[cur], L.red[cur ^ 1], L.black, om, w);
+      part += colour_phase<double, 2, RED, DO_RELAX | DO_RES, !GRID>(L, L.red[cur], L.red[cur ^ 1], L.black, om, w);
       share<GRID>(part, l & 1, sh, a.partial);
       barrier();
       if (dig == 0) {
@@ -704,13 +704,13 @@ __device__ __forceinline__ double smooth(const SPArgs &a, int level, int &cur, b
     }
     cur ^= 1;
     if (l < nr || need_res)
-      part = colour_phase<double, 2, BLACK, DO_RELAX | DO_RES>(L, L.black, L.black, L.red[cur], om, w);
+      part = colour_phase<double, 2, BLACK, DO_RELAX | DO_RES, !GRID>(L, L.black, L.black, L.red[cur], om, w);
     else
-      colour_phase<double, 2, BLACK, DO_RELAX>(L, L.black, L.black, L.red[cur], om, w);
+      colour_phase<double, 2, BLACK, DO_RELAX, !GRID>(L, L.black, L.black, L.red[cur], om, w);
     barrier();
   }
   if (need_res && !stopped) {
-    part += colour_phase<double, 2, RED, DO_RES>(L, L.red[cur], nullptr, L.black, om, w);
+    part += colour_phase<double, 2, RED, DO_RES, !GRID>(L, L.red[cur], nullptr, L.black, om, w);
     share<GRID>(part, 1, sh, a.partial);   // sweep 4 (l = 5)
     barrier();
     res = total<GRID>(1, sh, a.partial);
@@ -725,13 +725,13 @@ __device__ __forceinline__ void restrict_level(const SPArgs &a, int level, int c
   const Lev<double> &F = level_of<GRID>(a, level), &C = level_of<GRID>(a, level + 1);
   double *R = residual_red(F, cur);
   const Team w = GRID ? grid_team() : block_team();
-  residual_colour<double, 2, RED>(F, F.red[cur], F.black, R, w);
-  residual_colour<double, 2, BLACK>(F, F.black, F.red[cur], F.rf[BLACK], w);
+  residual_colour<double, 2, RED, !GRID>(F, F.red[cur], F.black, R, w);
+  residual_colour<double, 2, BLACK, !GRID>(F, F.black, F.red[cur], F.rf[BLACK], w);
   if (GRID)
     grid.sync();
   else
     __syncthreads();
-  restrict_to<double>(F, C, R, F.rf[BLACK], masks, true, a.omega, w);
+  restrict_to<double, !GRID>(F, C, R, F.rf[BLACK], masks, true, a.omega, w);
   if (GRID)
     grid.sync();
   else
@@ -773,7 +773,7 @@ __device__ __forceinline__ void chip_cycle(const SPArgs &a, bool first, int *ite
     if (g <= mid) cur[l] = 0;
     if (g > mid) {
       const Lev<double> &F = level_of<false>(a, l), &C = level_of<false>(a, l + 1);
-      prolong_to<double>(F, C, F.red[cur[l]], F.red[cur[l] ^ 1], C.red[cur[l + 1]], block_team());
+      prolong_to<double, true>(F, C, F.red[cur[l]], F.red[cur[l] ^ 1], C.red[cur[l + 1]], block_team());
       __syncthreads();
     }
     int k = 0;

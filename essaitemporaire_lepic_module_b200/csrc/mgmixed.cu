@@ -222,25 +222,25 @@ __device__ __forceinline__ void sweeps(const XArgs &a, const Lev &L, int nu, boo
     const bool last = s == nu - 1, add = GRID && addu && last;
     if (s > 0 || !started) {
       if (add)
-        colour_phase<float, XV, mgs::RED, DO_RELAX | DO_ADDU>(L, L.red[0], L.red[0], L.black, om, w, nullptr,
+        colour_phase<float, XV, mgs::RED, DO_RELAX | DO_ADDU, !GRID>(L, L.red[0], L.red[0], L.black, om, w, nullptr,
                                                               a.us[mgs::RED]);
       else
-        colour_phase<float, XV, mgs::RED, DO_RELAX>(L, L.red[0], L.red[0], L.black, om, w);
+        colour_phase<float, XV, mgs::RED, DO_RELAX, !GRID>(L, L.red[0], L.red[0], L.black, om, w);
       barrier<GRID>(grid);
     }
     if (s == 0 && started) {
       if (last && rf)
-        colour_phase<float, XV, mgs::BLACK, DO_RELAX | DO_RF | ZERO>(L, L.black, L.black, L.red[0], om, w,
+        colour_phase<float, XV, mgs::BLACK, DO_RELAX | DO_RF | ZERO, !GRID>(L, L.black, L.black, L.red[0], om, w,
                                                                      L.rf[mgs::BLACK]);
       else
-        colour_phase<float, XV, mgs::BLACK, DO_RELAX | ZERO>(L, L.black, L.black, L.red[0], om, w);
+        colour_phase<float, XV, mgs::BLACK, DO_RELAX | ZERO, !GRID>(L, L.black, L.black, L.red[0], om, w);
     } else if (last && rf) {
-      colour_phase<float, XV, mgs::BLACK, DO_RELAX | DO_RF>(L, L.black, L.black, L.red[0], om, w, L.rf[mgs::BLACK]);
+      colour_phase<float, XV, mgs::BLACK, DO_RELAX | DO_RF, !GRID>(L, L.black, L.black, L.red[0], om, w, L.rf[mgs::BLACK]);
     } else if (add) {
-      colour_phase<float, XV, mgs::BLACK, DO_RELAX | DO_ADDU>(L, L.black, L.black, L.red[0], om, w, nullptr,
+      colour_phase<float, XV, mgs::BLACK, DO_RELAX | DO_ADDU, !GRID>(L, L.black, L.black, L.red[0], om, w, nullptr,
                                                               a.us[mgs::BLACK]);
     } else {
-      colour_phase<float, XV, mgs::BLACK, DO_RELAX>(L, L.black, L.black, L.red[0], om, w);
+      colour_phase<float, XV, mgs::BLACK, DO_RELAX, !GRID>(L, L.black, L.black, L.red[0], om, w);
     }
     barrier<GRID>(grid);
   }
@@ -253,11 +253,11 @@ __device__ __forceinline__ void restrict_level(const XArgs &a, int l, bool swept
   using namespace mgs;
   const Team w = team<GRID>();
   const Lev &F = level_of<GRID>(a, l), &C = level_of<GRID>(a, l + 1);
-  residual_colour<float, XV, mgs::RED>(F, F.red[0], F.black, F.rf[mgs::RED], w);
-  if (!swept) residual_colour<float, XV, mgs::BLACK>(F, F.black, F.red[0], F.rf[mgs::BLACK], w);
+  residual_colour<float, XV, mgs::RED, !GRID>(F, F.red[0], F.black, F.rf[mgs::RED], w);
+  if (!swept) residual_colour<float, XV, mgs::BLACK, !GRID>(F, F.black, F.red[0], F.rf[mgs::BLACK], w);
   barrier<GRID>(grid);
   // (a level that is not swept on the way down starts from 0)
-  restrict_to<float>(F, C, F.rf[mgs::RED], F.rf[mgs::BLACK], masks, (l + 1 == a.ng ? a.coarse_sweeps : a.nu_pre) > 0,
+  restrict_to<float, !GRID>(F, C, F.rf[mgs::RED], F.rf[mgs::BLACK], masks, (l + 1 == a.ng ? a.coarse_sweeps : a.nu_pre) > 0,
                      a.omega, w);
   barrier<GRID>(grid);
 }
@@ -303,7 +303,7 @@ __device__ __forceinline__ void chip_cycle(const XArgs &a, bool first, Sync &gri
       if (g < mid) restrict_level<false>(a, l, a.nu_pre > 0, first, grid);
     } else {
       const Lev &F = level_of<false>(a, l), &C = level_of<false>(a, l + 1);
-      prolong_to<float>(F, C, F.red[0], nullptr, C.red[0], block_team());
+      prolong_to<float, true>(F, C, F.red[0], nullptr, C.red[0], block_team());
       __syncthreads();
       sweeps<false>(a, F, a.nu_post, false, false, false, grid);
     }
