@@ -124,6 +124,7 @@ struct Tile {
   const unsigned char *cw;    // all-wall flags of the box cells
   int bx, by, bz;             // grid coordinates of box node (0,0,0)
   const float4 *B;            // B map at the box nodes (map on the node grid)
+  bool inner;                 // every cell of the box is a cell 1..n
 };
 
 // sum of k_i e_i, i = 0..7, rounded as a chain of multiply-adds in order
@@ -341,7 +342,9 @@ __device__ __forceinline__ void push_quad(const Dims &d, const MixedConst &c, co
       continue;
     }
     const int ix = (cc & CM) + 1, iy = ((cc >> CB) & CM) + 1, iz = (cc >> (2 * CB)) + 1;
-    if (cc < 0 || ix > n1 || iy > n2 || iz > n3) {
+    int lx, ly, lz;
+    const bool boxed = in_box<PushBox>(T, ix, iy, iz, lx, ly, lz);
+    if (!(boxed && T.inner) && (cc < 0 || ix > n1 || iy > n2 || iz > n3)) {
       raise_err(err, LEPIC_ERR_CELL, (int)(i0 + k));
       hole[k] = true;
       continue;
@@ -356,8 +359,6 @@ __device__ __forceinline__ void push_quad(const Dims &d, const MixedConst &c, co
     // loads on 32-bit addresses), else from HBM
     long long g0, sy, sz;
     float4 e0, e1, e2, e3, e4, e5, e6, e7;
-    int lx, ly, lz;
-    const bool boxed = in_box<PushBox>(T, ix, iy, iz, lx, ly, lz);
     if (boxed) {
       g0 = lx + TN * (ly + TN * lz);
       sy = TN;
@@ -417,86 +418,88 @@ __device__ __forceinline__ void push_quad(const Dims &d, const MixedConst &c, co
     fx = fx + vx * c.dth0;
     fy = fy + vy * c.dth1;
     fz = fz + vz * c.dth2;
-    int sx = 0, syi = 0, szi = 0;
-    if (!(fx >= 0.f && fx < 1.f)) {
-      sx = __float2int_rd(fx);
-      fx -= (float)sx;
-      if (fx >= 1.f) { fx = 0.f; sx += 1; }
-    }
-    if (!(fy >= 0.f && fy < 1.f)) {
-      syi = __float2int_rd(fy);
-      fy -= (float)syi;
-      if (fy >= 1.f) { fy = 0.f; syi += 1; }
-    }
-    if (!(fz >= 0.f && fz < 1.f)) {
-      szi = __float2int_rd(fz);
-      fz -= (float)szi;
-      if (fz >= 1.f) { fz = 0.f; szi += 1; }
-    }
-    int ax = ix + sx, ay = iy + syi, az = iz + szi;
-    int cx = ax, cy = ay, cz = az;
-    bool lost = false;
-    if (sx | syi | szi) {
-      // a new cell: the loss test on the clamped cell before any periodic
-      // wrap, as Src/part_expmover.f90:250-275 (the cell a particle stays in
-      // passed the test when the particle entered it), then the wrap of the
-      // particles that stay (:460-465)
-      cx = ax < 0 ? 0 : (ax > n1 + 1 ? n1 + 1 : ax);
-      cy = ay < 0 ? 0 : (ay > n2 + 1 ? n2 + 1 : ay);
-      cz = az < 0 ? 0 : (az > n3 + 1 ? n3 + 1 : az);
-      int lx, ly, lz;
-      const bool wall = in_box<PushBox>(T, cx, cy, cz, lx, ly, lz) ? T.cw[lx + (TN - 1) * (ly + (TN - 1) * lz)] != 0
-                                                          : cw[d.c(cx, cy, cz)] != 0;
-      if (c.flag_nmn == 1 && ax < 1 && !wall) {
-        // specular reflection at the Neumann plane x = 0 (Src/part_expmover.f90:
-        // 437-446): x = (ax - 1 + fx) h < 0 becomes -x, vx changes sign
-        const float g = 1.f - fx;
-        ax = 1 - ax;
-        if (g >= 1.f) {
-          fx = 0.f;
-          ax += 1;
-        } else {
-          fx = g;
-        }
-        vx = -vx;
+    int ax = ix, ay = iy, az = iz;
+    if (!(fminf(fminf(fx, fy), fz) >= 0.f && fmaxf(fmaxf(fx, fy), fz) < 1.f)) {
+      int sx = 0, syi = 0, szi = 0;
+      if (!(fx >= 0.f && fx < 1.f)) {
+        sx = __float2int_rd(fx);
+        fx -= (float)sx;
+        if (fx >= 1.f) { fx = 0.f; sx += 1; }
       }
-      lost = wall || ax < 1 || ax > n1;
-      if (c.flag_pbc == 1) {
-        if (!lost) {
-          if (ay > n2) ay -= n2;
-          if (ay < 1) ay += n2;
-          if (az > n3) az -= n3;
-          if (az < 1) az += n3;
-        }
-      } else {
-        lost = lost || ay < 1 || ay > n2 || az < 1 || az > n3;
+      if (!(fy >= 0.f && fy < 1.f)) {
+        syi = __float2int_rd(fy);
+        fy -= (float)syi;
+        if (fy >= 1.f) { fy = 0.f; syi += 1; }
       }
-    }
-    if (lost) {
-      // lost at a wall (Src/part_expmover.f90:275-433): every cell outside
-      // 1..n has only wall nodes in a closed box; a cell inside 1..n is lost
-      // when all of its 8 nodes are walls
-      const double Eki = 0.5 * c.Nm * c.mass * ((double)vx * vx + (double)vy * vy + (double)vz * vz);
-      const int igrid = bcnd[d.g(cx, cy, cz)];
-      atomicAdd(&acc[0], Eki);
-      if (igrid >= 0 && igrid <= c.ngrid) {
-        atomicAdd(&acc[2 + 2 * igrid], 1.0);
-        atomicAdd(&acc[3 + 2 * igrid], Eki);
-        if (DIE) {
-          // periodic planes: z wraps for the wall charge, y does not
-          // (Src/part_expmover.f90:306-316)
-          int aw = az, cw_z = cz;
-          if (c.flag_pbc == 1 && (az > n3 || az < 1)) {
-            aw = az > n3 ? az - n3 : az + n3;
-            cw_z = aw < 0 ? 0 : (aw > n3 + 1 ? n3 + 1 : aw);
+      if (!(fz >= 0.f && fz < 1.f)) {
+        szi = __float2int_rd(fz);
+        fz -= (float)szi;
+        if (fz >= 1.f) { fz = 0.f; szi += 1; }
+      }
+      if (sx | syi | szi) {
+        ax = ix + sx, ay = iy + syi, az = iz + szi;
+        // a new cell: the loss test on the clamped cell before any periodic
+        // wrap, as Src/part_expmover.f90:250-275 (the cell a particle stays in
+        // passed the test when the particle entered it), then the wrap of the
+        // particles that stay (:460-465)
+        const int cx = ax < 0 ? 0 : (ax > n1 + 1 ? n1 + 1 : ax);
+        const int cy = ay < 0 ? 0 : (ay > n2 + 1 ? n2 + 1 : ay);
+        const int cz = az < 0 ? 0 : (az > n3 + 1 ? n3 + 1 : az);
+        const bool wall = in_box<PushBox>(T, cx, cy, cz, lx, ly, lz) ? T.cw[lx + (TN - 1) * (ly + (TN - 1) * lz)] != 0
+                                                            : cw[d.c(cx, cy, cz)] != 0;
+        if (c.flag_nmn == 1 && ax < 1 && !wall) {
+          // specular reflection at the Neumann plane x = 0 (Src/part_expmover.f90:
+          // 437-446): x = (ax - 1 + fx) h < 0 becomes -x, vx changes sign
+          const float g = 1.f - fx;
+          ax = 1 - ax;
+          if (g >= 1.f) {
+            fx = 0.f;
+            ax += 1;
+          } else {
+            fx = g;
           }
-          const Dielectric die = {c.die.dtype, c.die.qxz, c.die.qyz, c.die.k3};
-          dielectric_charge_cells(die, d.N1, d.N2, igrid, ax, ay, aw, fx, fy, fz, cx, cy, cw_z);
+          vx = -vx;
+        }
+        bool lost = wall || ax < 1 || ax > n1;
+        if (c.flag_pbc == 1) {
+          if (!lost) {
+            if (ay > n2) ay -= n2;
+            if (ay < 1) ay += n2;
+            if (az > n3) az -= n3;
+            if (az < 1) az += n3;
+          }
+        } else {
+          lost = lost || ay < 1 || ay > n2 || az < 1 || az > n3;
+        }
+        if (lost) {
+          // lost at a wall (Src/part_expmover.f90:275-433): every cell outside
+          // 1..n has only wall nodes in a closed box; a cell inside 1..n is lost
+          // when all of its 8 nodes are walls
+          const double Eki = 0.5 * c.Nm * c.mass * ((double)vx * vx + (double)vy * vy + (double)vz * vz);
+          const int igrid = bcnd[d.g(cx, cy, cz)];
+          atomicAdd(&acc[0], Eki);
+          if (igrid >= 0 && igrid <= c.ngrid) {
+            atomicAdd(&acc[2 + 2 * igrid], 1.0);
+            atomicAdd(&acc[3 + 2 * igrid], Eki);
+            if (DIE) {
+              // periodic planes: z wraps for the wall charge, y does not
+              // (Src/part_expmover.f90:306-316)
+              int aw = az, cw_z = cz;
+              if (c.flag_pbc == 1 && (az > n3 || az < 1)) {
+                aw = az > n3 ? az - n3 : az + n3;
+                cw_z = aw < 0 ? 0 : (aw > n3 + 1 ? n3 + 1 : aw);
+              }
+              const Dielectric die = {c.die.dtype, c.die.qxz, c.die.qyz, c.die.k3};
+              dielectric_charge_cells(die, d.N1, d.N2, igrid, ax, ay, aw, fx, fy, fz, cx, cy, cw_z);
+            }
+          }
+          hole[k] = true;
+        } else {
+          (&c4.x)[k] = (ax - 1) | (ay - 1) << CB | (az - 1) << (2 * CB);
         }
       }
-      hole[k] = true;
-    } else {
-      (&c4.x)[k] = (ax - 1) | (ay - 1) << CB | (az - 1) << (2 * CB);
+    }
+    if (DEP && !hole[k]) {
       jx[k] = ax;
       jy[k] = ay;
       jz[k] = az;
@@ -620,7 +623,9 @@ __global__ void __launch_bounds__(MBK, 3) k_push_tiles(
   long long lo, hi;
   part_range(tile_off, *count, blockIdx.x, PUSH_PARTS, t, lo, hi);
   const int tx = t % c.ntx, ty = (t / c.ntx) % c.nty, tz = t / (c.ntx * c.nty);
-  const Tile T{nullptr, s_E, s_cw, tx * TC + 1 - TH, ty * TC + 1 - TH, tz * TC + 1 - TH, s_B};
+  const Tile T{nullptr, s_E, s_cw, tx * TC + 1 - TH, ty * TC + 1 - TH, tz * TC + 1 - TH, s_B,
+               tx > 0 && ty > 0 && tz > 0 && tx * TC + TN - TH <= d.n1 + 1 && ty * TC + TN - TH <= d.n2 + 1 &&
+                   tz * TC + TN - TH <= d.n3 + 1};
   const long long first = lo & ~3LL;
   // the copies of this thread's quad at i0 (i0 < hi: i0 + 3 < cap, 16-byte
   // aligned as i0 is a multiple of 4)
@@ -706,7 +711,7 @@ __global__ void __launch_bounds__(MBK, 5) k_deposit_tiles(Dims d, int ntx, int n
   long long lo, hi;
   part_range(tile_off, *count, blockIdx.x, parts, t, lo, hi);
   const int tx = t % ntx, ty = (t / ntx) % nty, tz = t / (ntx * nty);
-  const Tile T{s_acc, nullptr, nullptr, tx * TC + 1 - TH, ty * TC + 1 - TH, tz * TC + 1 - TH, nullptr};
+  const Tile T{s_acc, nullptr, nullptr, tx * TC + 1 - TH, ty * TC + 1 - TH, tz * TC + 1 - TH, nullptr, false};
   // the window at `base` (a multiple of 4, as cap is): 16-byte copies of the
   // 4-byte planes, 4-byte ones of the flags (whose address is only that
   // aligned)
@@ -753,7 +758,7 @@ __global__ void __launch_bounds__(MBK, 3) k_push_deposit_tail(
     const double *__restrict__ kq, double *__restrict__ np, int *__restrict__ holes, int *__restrict__ nholes,
     double *__restrict__ acc, int *__restrict__ err) {
   acc = my_losses(acc, c.ngrid);
-  const Tile T{nullptr, nullptr, nullptr, 0, 0, 0, nullptr};
+  const Tile T{nullptr, nullptr, nullptr, 0, 0, 0, nullptr, false};
   const long long N = *count;
   const long long lo = tile_off ? tile_off[c.ntiles] : 0;
   const long long first = lo & ~3LL;
@@ -1086,7 +1091,7 @@ __global__ void k_deposit_mixed(Dims d, double kdep, const int *__restrict__ cel
   }
   int w[8];
   qweights(p[i], p[cap + i], p[2 * cap + i], w);
-  const Tile T{nullptr, nullptr, nullptr, 0, 0, 0, nullptr};
+  const Tile T{nullptr, nullptr, nullptr, 0, 0, 0, nullptr, false};
   deposit8(d, T, ix, iy, iz, w, kdep, kq, np);
 }
 
