@@ -951,7 +951,7 @@ int launch_split(const int n[3], const double h[3], double *u, const double *b, 
                  cudaStream_t s, bool &launched) {
   using Lev = mgs::Lev<double>;
   launched = false;
-  if (Lev::elements(n[0], n[1], n[2]) >= 1200000000LL) return LEPIC_OK;
+  if (Lev::elements(n[0], n[1], n[2]) >= 2130000000LL) return LEPIC_OK;
   SPArgs A;
   memset(&A, 0, sizeof(A));
   A.ng = ng;

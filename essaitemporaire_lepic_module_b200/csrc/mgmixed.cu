@@ -456,7 +456,7 @@ int launch_pdesolver_mixed(const Dims &d, const double h[3], double *u, const do
   A.barrier = grid_barrier();
   A.err = c.d_err;
   if (!A.barrier) return LEPIC_ERR_CUDA;
-  if (Lev::elements(n[0], n[1], n[2]) >= 1200000000LL) return LEPIC_ERR_UNSUPPORTED;   // 32-bit element numbers
+  if (Lev::elements(n[0], n[1], n[2]) >= 2130000000LL) return LEPIC_ERR_UNSUPPORTED;   // 32-bit element numbers
   // shapes and coefficients per level (Src/mg.h)
   for (int l = 1; l <= ng; ++l) {
     double hl[3];
