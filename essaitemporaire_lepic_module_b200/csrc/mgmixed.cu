@@ -49,8 +49,9 @@ using Lev = mgs::Lev<float>;
 
 constexpr int XM_MAX = 13;      // multigrid levels
 // threads per block: twice as many, at half the registers, on grids whose
-// finest level moves through HBM (a solve at 256^3: 13.9 -> 12.7 ms; at 192^3
-// and 176^3 the same; at 160^3 10.4 -> 11.3 ms, at 128^3 617 -> 714 us)
+// finest level moves through HBM (a solve, with the cooperative groups'
+// barrier: 256^3 13.9 -> 12.7 ms, 192^3 and 176^3 the same, 160^3 10.4 -> 11.3
+// ms, 128^3 617 -> 714 us)
 constexpr int XM_BLOCK = 512, XM_BLOCK_LARGE = 1024;
 constexpr long long XM_LARGE = 3000000;   // elements per colour from which it takes those
 constexpr int XV = 4;           // elements per 16-byte load

@@ -22,8 +22,6 @@
 // the written buffer is simply not taken.
 #pragma once
 
-#include <cooperative_groups.h>
-
 #include <type_traits>
 
 #include "lepic_internal.cuh"
@@ -89,7 +87,7 @@ struct Lev {
 
 // The barrier between two phases of the levels on the grid: of all blocks of a
 // cooperative launch, or, for small grids, of one cluster of CLUSTER blocks
-// (0.3 against 1.2 us by itself, and a phase's stores reach only as far).
+// (0.3 us by itself, the cooperative groups' barrier of the grid 1.2).
 // The grid's barrier is a word of its own per launch (grid_barrier()): each
 // block adds 1, block 0 what takes the word to its top bit flipped and the
 // count back to where it was, and the blocks watch that bit.  Unlike the

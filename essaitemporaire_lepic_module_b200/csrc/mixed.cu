@@ -418,6 +418,10 @@ __device__ __forceinline__ void push_quad(const Dims &d, const MixedConst &c, co
     fx = fx + vx * c.dth0;
     fy = fy + vy * c.dth1;
     fz = fz + vz * c.dth2;
+    // most particles stay in their cell: one test for the three axes, and
+    // neither loss test nor repacking behind it (with a test per axis 136
+    // instead of 131 us per 1.05e7 particles at 48x80x112; a NaN, which the
+    // minimum skips, keeps its cell either way)
     int ax = ix, ay = iy, az = iz;
     if (!(fminf(fminf(fx, fy), fz) >= 0.f && fmaxf(fmaxf(fx, fy), fz) < 1.f)) {
       int sx = 0, syi = 0, szi = 0;
