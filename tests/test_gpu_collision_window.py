@@ -17,9 +17,10 @@ Bars:
   * the mixed-precision adjoint (FP32 particles and pushes, FP32 V-cycles in
     FP64 refinement) against the FP64 adjoint for all three observables
     (energy, probe potential, wall energy flux): J, dJ/dV and dJ/dB_z within
-    1e-4 (dJ/dB_z of the wall flux within 1e-3), the directional derivative
-    in the initial velocities within 2e-4 (particles whose wall crossing
-    differs between the FP32 and FP64 windows move these by up to a few 1e-4);
+    1e-4 (dJ/dB_z of the wall flux within 1e-3), the gradient in the initial
+    velocities within 8e-6 in the 2-norm, but for at most 1e-4 of the
+    particles (whose wall crossing differs between the two windows, or whose
+    replayed ionization is just above its threshold);
   * the torch.autograd.Function returns the window's own gradients.
 """
 import dataclasses
@@ -121,7 +122,6 @@ def test_fp64_adjoint_vs_central_differences(windows, observable):
 
 @pytest.mark.parametrize("observable", ["energy", "probe", "flux"])
 def test_mixed_adjoint_vs_fp64_adjoint(windows, observable):
-    import torch
     _, w32, w64, V, Bz = windows
     J32 = w32.forward(V, Bz, observable=observable)
     g32 = w32.backward()
@@ -135,12 +135,19 @@ def test_mixed_adjoint_vs_fp64_adjoint(windows, observable):
     # typically 1e-6), so that derivative is held to 1e-3
     rel_bz = 1e-3 if observable == "flux" else 1e-4
     assert _close(g32[1], g64[1], rel_bz), (g32[1], g64[1])
-    # a directional derivative in the initial velocities sums over every
-    # particle, those whose wall crossing differs between the windows included:
-    # it has agreed to 1e-6 .. 1e-4 over the runs, so it is held to 2e-4
-    torch.manual_seed(1)
-    dv = torch.randn(g64[2].shape, dtype=torch.float64, device="cuda")
-    assert _close(float((g32[2] * dv).sum()), float((g64[2] * dv).sum()), 2e-4)
+    # the gradient in the initial velocities, particle by particle: FP32
+    # rounding through the window leaves the 2-norm of the difference at 2e-7
+    # to 6e-7 of the gradient's.  A few of the 247,000 particles are further
+    # off: one that reaches a wall in one window and not in the other (one run
+    # of twelve; by 0.6 of the rms, which is as much as 2 % of the derivative
+    # along a random direction, whose terms cancel), or one whose replayed
+    # ionization is just above its threshold.  Those off by more than 1e-3 of
+    # the rms are counted instead (at most 1e-4 of all); the rest holds 6e-7
+    # and twelve just below that line, 1e-3 sqrt(12 / 247,000) = 7e-6.
+    n = g64[2].shape[1]
+    off = (g32[2] - g64[2]).norm(dim=0) > 1e-3 * g64[2].norm() / n ** 0.5
+    assert int(off.sum()) <= 1e-4 * n, int(off.sum())
+    assert float((g32[2] - g64[2])[:, ~off].norm()) <= 8e-6 * float(g64[2].norm())
     # backward no dearer than 3 forward passes of the window
     assert w32.timing["backward_ms"] <= 3.0 * w32.timing["forward_ms"] + 5.0
 
