@@ -51,9 +51,9 @@ int check_err(cudaStream_t s);                  // sync, read + clear device err
 // saves two staged copies of about 8 us each); nullptr when there is none.
 constexpr int RESULT_WORDS = 8;
 double *result_block();
-// A barrier word for one launch of a kernel over the whole device, in device
-// memory and in the state every launch leaves behind.  They are handed out in
-// turn, so launches that overlap have different ones.
+// A line of words for the barrier of one launch of a kernel over the whole
+// device, in device memory and in the state every launch leaves behind.  They
+// are handed out in turn, so launches that overlap have different ones.
 unsigned *grid_barrier();
 int timer_start(const char *name, cudaStream_t s);  // -1 when timing is off
 void timer_stop(int id, cudaStream_t s);

@@ -692,6 +692,7 @@ __device__ __forceinline__ double smooth(const SPArgs &a, int level, int &cur, b
       if (dig == 0) {
         res = total<GRID>(l & 1, sh, a.partial);
         stopped = res <= eps_abs;
+        if (!GRID && l % SWEEPS_PER_BEAT == 0) grid.beat();
       } else if (l >= 3) {
         const double before = l == 3 ? total<GRID>((l - 1) & 1, sh, a.partial) : res;
         res = total<GRID>(l & 1, sh, a.partial);

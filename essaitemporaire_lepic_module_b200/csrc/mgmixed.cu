@@ -221,6 +221,7 @@ __device__ __forceinline__ void sweeps(const XArgs &a, const Lev &L, int nu, boo
   const float om = a.omega;
   for (int s = 0; s < nu; ++s) {
     const bool last = s == nu - 1, add = GRID && addu && last;
+    if (!GRID && s % SWEEPS_PER_BEAT == SWEEPS_PER_BEAT - 1) grid.beat();
     if (s > 0 || !started) {
       if (add)
         colour_phase<float, XV, mgs::RED, DO_RELAX | DO_ADDU, !GRID>(L, L.red[0], L.red[0], L.black, om, w, nullptr,

@@ -95,14 +95,23 @@ struct Lev {
 // read that sees the bit is the acquire (with relaxed reads and a fence behind
 // them the mixed solve of 48x40x56 took 468 us instead of 421).  Solves at
 // 128^3: FP64 4.32 -> 4.07 ms, mixed 613 -> 582 us; at 256^3 mixed 12.4 -> 11.2
-// ms.  The blocks are co-resident (cooperative launch), so the wait ends;
-// should one not, the block records LEPIC_ERR_TIMEOUT after about a second and
-// waits no more.
+// ms.  The blocks are co-resident (cooperative launch) and a phase takes
+// milliseconds at most, but for block 0's on the levels on chip, which may
+// smooth the coarsest one a million times: it counts its sweeps there in a
+// second word (beat).  A wait therefore lasts as long as anything moves,
+// arrivals or beats; where nothing has for BARRIER_ROUNDS rounds of looks (one
+// and a half seconds; counted in looks, since a process that shares the
+// device may stop this one for any time), the block records LEPIC_ERR_TIMEOUT
+// and waits no more.
+constexpr unsigned BARRIER_LOOKS = 1u << 12, BARRIER_ROUNDS = 1u << 10;
+constexpr int SWEEPS_PER_BEAT = 256;
 struct GridSync {
+  enum { WORD = 0, BEAT = 1 };   // of the launch's line
   struct State {
-    unsigned *word, phase;
+    unsigned *line, phase;
     int *err;
     bool dead;
+    unsigned moved, idle;   // what had moved after the last round, rounds without any since
   };
   static __device__ __forceinline__ State &state() {
     __shared__ State s;
@@ -114,31 +123,55 @@ struct GridSync {
     return v;
   }
   // (the bit cannot flip before this block has arrived once)
-  __device__ GridSync(unsigned *word, int *err) {
-    if (threadIdx.x == 0) state() = {word, look(word) & 0x80000000u, err, false};
+  __device__ GridSync(unsigned *line, int *err) {
+    if (threadIdx.x == 0) state() = {line, look(line + WORD) & 0x80000000u, err, false, 0, 0};
+  }
+  // looks at `word` until its top bit differs from phase's, BARRIER_LOOKS
+  // times at most: what is left of them (a loop of its own instructions: with
+  // the compiler's, the rest of the wait costs every barrier of a solve 1 %)
+  static __device__ __forceinline__ unsigned watch(const unsigned *word, unsigned phase) {
+    unsigned left;
+    asm volatile(
+        "{\n .reg .pred p;\n .reg .b32 v, n;\n mov.u32 n, %3;\n"
+        "LOOK%=:\n ld.acquire.gpu.global.u32 v, [%1];\n xor.b32 v, v, %2;\n setp.lt.s32 p, v, 0;\n"
+        " @p bra SEEN%=;\n sub.u32 n, n, 1;\n setp.ne.u32 p, n, 0;\n @p bra LOOK%=;\n"
+        "SEEN%=:\n mov.u32 %0, n;\n}\n"
+        : "=r"(left)
+        : "l"(word), "r"(phase), "n"(BARRIER_LOOKS)
+        : "memory");
+    return left;
+  }
+  // after a round of looks: nothing has moved for too long
+  static __device__ __forceinline__ bool give_up(State &s) {
+    const unsigned moved = look(s.line + WORD) + look(s.line + BEAT);
+    s.idle = moved != s.moved ? 0 : s.idle + 1;
+    s.moved = moved;
+    if (s.idle < BARRIER_ROUNDS) return false;
+    s.dead = true;
+    raise_err(s.err, LEPIC_ERR_TIMEOUT, (int)blockIdx.x);
+    return true;
   }
   __device__ __forceinline__ void sync() {
     __syncthreads();
     if (threadIdx.x == 0) {
       State &s = state();
       const unsigned add = blockIdx.x == 0 ? 0x80000000u - (gridDim.x - 1) : 1u;
-      asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(s.word), "r"(add) : "memory");
-      if (!s.dead) {
-        int tries = 1 << 22;
-        while (((look(s.word) ^ s.phase) & 0x80000000u) == 0 && --tries) {
+      asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(s.line + WORD), "r"(add) : "memory");
+      if (!s.dead)
+        while (!watch(s.line + WORD, s.phase) && !give_up(s)) {
         }
-        if (!tries) {
-          s.dead = true;
-          raise_err(s.err, LEPIC_ERR_TIMEOUT, (int)blockIdx.x);
-        }
-      }
       s.phase ^= 0x80000000u;
     }
     __syncthreads();
   }
+  // block 0 on the levels on chip: the others' wait goes on
+  __device__ __forceinline__ void beat() {
+    if (threadIdx.x == 0) asm volatile("red.relaxed.gpu.global.add.u32 [%0], 1;" ::"l"(state().line + BEAT));
+  }
 };
 struct ClusterSync {
   __device__ ClusterSync(unsigned *, int *) {}
+  __device__ __forceinline__ void beat() {}
   __device__ __forceinline__ void sync() {
     asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
   }

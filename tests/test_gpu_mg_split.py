@@ -98,3 +98,61 @@ def test_mixed_schedules_reach_the_fp64_solution(n, ng, nu):
     assert rc == 0
     assert float((a - b).abs().max()) <= 1e-6 * float(b.abs().max())
     assert bool((a[bct > 0] == torch.as_tensor(phi0, device=dev)[bct > 0]).all())
+
+
+def test_the_grid_waits_for_a_million_sweeps_on_chip():
+    """A tolerance that rounding never reaches: the coarsest level, on chip in
+    block 0 while every other block waits in one barrier, is swept as often as
+    the schedule allows, for seconds.  FP64 against the general kernel with
+    the coarsest level solved to 1e-14 (its residual over alpha; phi is then
+    off by at most 1e-11 times that level's condition number of a few
+    hundred); mixed, as many sweeps on request, against few, where the FP32
+    coarse solution is the same to its rounding.  No status is recorded."""
+    import time
+
+    import torch
+    from essaitemporaire_lepic_module_b200 import config
+    from essaitemporaire_lepic_module_b200._lib import LepicGrid, lib, phys_struct
+
+    st = config.build("box16")
+    n, ng = (64, 64, 64), 3                       # 67,000 elements per colour, 16^3 on chip
+    shape = tuple(v + 3 for v in n)
+    bc = np.ones(shape, dtype=np.int32)
+    bc[2:-2, 2:-2, 2:-2] = -1
+    dev = torch.device("cuda")
+    bct = torch.as_tensor(bc, device=dev)
+    phi0 = torch.as_tensor(np.where(bc > 0, 1.0, 0.0), device=dev)
+    rt = torch.as_tensor(np.random.default_rng(5).normal(size=tuple(v - 1 for v in shape)) * 1e-5, device=dev)
+    grid = LepicGrid()
+    for a in range(3):
+        grid.n[a], grid.h[a] = n[a], 1.0e-4
+    grid.bcnd = bct.data_ptr()
+    P = phys_struct(st)
+    L, s = lib(), C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    took, got = [], []
+    for entry, eps in ((L.lepic_dev_pdesolver, 0.0), (L.lepic_dev_pdesolver_noalloc, 1e-14)):
+        phi = phi0.clone()
+        k, kt, res = C.c_int(0), C.c_double(0), C.c_double(0)
+        t0 = time.perf_counter()
+        rc = entry(C.byref(grid), C.c_void_p(phi.data_ptr()), C.c_void_p(rt.data_ptr()), 1, eps, 1.4, ng,
+                   C.byref(P), C.byref(k), C.byref(kt), C.byref(res), s)
+        took.append(time.perf_counter() - t0)
+        assert rc == 0
+        got.append((kt.value, phi))
+    print("seconds: split, general", took)
+    assert got[0][0] >= 1000000 / 16 > got[1][0]
+    assert float((got[0][1] - got[1][1]).abs().max()) <= 1e-8 * float(got[1][1].abs().max())
+    phis = []
+    for sweeps in (2000, 3000000):
+        phi = phi0.clone()
+        it, res = C.c_int(0), C.c_double(0)
+        t0 = time.perf_counter()
+        rc = L.lepic_dev_pdesolver_mixed(C.byref(grid), C.c_void_p(phi.data_ptr()), C.c_void_p(rt.data_ptr()), 1e-30,
+                                         1.3, ng, C.byref(P), 1, 1, 3, 2, 2, sweeps, C.byref(it), C.byref(res), s)
+        took.append(time.perf_counter() - t0)
+        assert rc == 23 and it.value == 1         # one refinement, not converged
+        phis.append(phi)
+    print("seconds: mixed", took[2:])
+    assert float((phis[0] - phis[1]).abs().max()) <= 1e-5 * float(phis[0].abs().max())
+    detail = C.c_int(0)
+    assert L.lepic_dev_check(s, C.byref(detail)) == 0
