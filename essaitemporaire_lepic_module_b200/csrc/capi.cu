@@ -299,6 +299,17 @@ int lepic_dev_wait_selftest(long long limit_ns, void *stream) {
   return LEPIC_OK;
 }
 
+int lepic_dev_solve_selftest(const lepic_grid_t *g, double *u, const double *b, int ng, const lepic_phys_t *P,
+                             int mixed, int wait, void *stream) {
+  if (!g || !P || P->flag_pbc || P->flag_nmn) return LEPIC_ERR_ARG;
+  if (!mixed)
+    return launch_pdesolver(Dims(g->n), g->h, u, b, g->bcnd, 1, 0.0, 1.4, ng, P->eps0, nullptr, nullptr, nullptr,
+                            S(stream), 0, 0, 0);
+  int it = 0;
+  return launch_pdesolver_mixed(Dims(g->n), g->h, u, b, g->bcnd, 0.0, 1.3, ng, P->eps0, 1, 1, 3, 2, 2, 20000,
+                                wait ? &it : nullptr, nullptr, S(stream), 0);
+}
+
 int lepic_dev_check_async(void *stream, int *host) {
   if (!host) return LEPIC_ERR_ARG;
   Ctx &c = ctx();

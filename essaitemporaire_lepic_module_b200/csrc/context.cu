@@ -45,13 +45,14 @@ Ctx &ctx() {
       cudaMemset(c.d_barrier, 0, BARRIERS * BARRIER_WORDS * sizeof(unsigned));
     else
       c.d_barrier = nullptr;
+    cudaStreamSynchronize(nullptr);   // a first launch on any stream finds them cleared
   }
   return c;
 }
 
-unsigned *grid_barrier() {
+GridBarrier grid_barrier(unsigned rounds) {
   Ctx &c = ctx();
-  return c.d_barrier ? c.d_barrier + (g_barrier++ % BARRIERS) * BARRIER_WORDS : nullptr;
+  return {c.d_barrier ? c.d_barrier + (g_barrier++ % BARRIERS) * BARRIER_WORDS : nullptr, rounds};
 }
 
 void *scratch(const char *name, size_t bytes) {
@@ -107,9 +108,6 @@ int check_err(cudaStream_t s) {
   if (code) {
     fprintf(stderr, "lepic_gpu: device status %d (detail %d)\n", code, c.h_err[1]);
     cudaMemsetAsync(c.d_err, 0, 2 * sizeof(int), s);
-    // a barrier that was given up has left its word between two states
-    if (code == LEPIC_ERR_TIMEOUT && c.d_barrier)
-      cudaMemsetAsync(c.d_barrier, 0, BARRIERS * BARRIER_WORDS * sizeof(unsigned), s);
     cudaStreamSynchronize(s);
   }
   return code;

@@ -40,7 +40,7 @@ struct Ctx {
   int sms = 0;
   int *d_err = nullptr;       // device int[2]
   int *h_err = nullptr;       // pinned host int[2]
-  unsigned *d_barrier = nullptr;   // the words of grid_barrier()
+  unsigned *d_barrier = nullptr;   // the lines of grid_barrier()
   cudaDeviceProp prop{};
 };
 Ctx &ctx();                                     // context of the current device
@@ -51,10 +51,16 @@ int check_err(cudaStream_t s);                  // sync, read + clear device err
 // saves two staged copies of about 8 us each); nullptr when there is none.
 constexpr int RESULT_WORDS = 8;
 double *result_block();
-// A line of words for the barrier of one launch of a kernel over the whole
-// device, in device memory and in the state every launch leaves behind.  They
-// are handed out in turn, so launches that overlap have different ones.
-unsigned *grid_barrier();
+// The barrier of one launch of a kernel over the whole device: a line of words
+// in device memory, in the state every launch leaves behind (they are handed
+// out in turn, so launches that overlap have different ones; nullptr: none),
+// and for how many rounds of looks a block waits while nothing moves.
+struct GridBarrier {
+  unsigned *line;
+  unsigned rounds;
+};
+constexpr unsigned BARRIER_ROUNDS = 1u << 10;
+GridBarrier grid_barrier(unsigned rounds = BARRIER_ROUNDS);
 int timer_start(const char *name, cudaStream_t s);  // -1 when timing is off
 void timer_stop(int id, cudaStream_t s);
 int cuda_status(cudaError_t e, const char *what);
@@ -258,7 +264,7 @@ int launch_cell_wall(const Dims &d, const int *bcnd, unsigned char *cw, cudaStre
 // pbc: periodic planes in y and z (bcnd 0); nmn: Neumann plane at x = 0 (bcnd -2)
 int launch_pdesolver(const Dims &d, const double h[3], double *u, const double *b, const int *bcnd,
                      int ncycl, double eps, double omega, int ng, double eps0, int *k, double *ktot,
-                     double *res, cudaStream_t s, int pbc = 0, int nmn = 0);
+                     double *res, cudaStream_t s, int pbc = 0, int nmn = 0, unsigned rounds = BARRIER_ROUNDS);
 // particles.cu
 // The drop-in mover's negative-ion bookkeeping (species tag_neg: flag_cex in
 // slot order in cex, compacted into cex_out; device counters cnt_cex[3],
@@ -329,7 +335,7 @@ int launch_sort_mixed(const lepic_grid_t &g, lepic_species_mixed_t &sp, int n_hi
 int launch_pdesolver_mixed(const Dims &d, const double h[3], double *u, const double *b, const int *bcnd,
                            double eps, double omega, int ng, double eps0, int max_refine, int nu_fine_pre,
                            int nu_fine_post, int nu_pre, int nu_post, int coarse_sweeps, int *iters,
-                           double *res_out, cudaStream_t s);
+                           double *res_out, cudaStream_t s, unsigned rounds = BARRIER_ROUNDS);
 
 // heating.cu (e or m: the electrons in one of the two layouts)
 int launch_eheating(const lepic_grid_t &g, lepic_species_f64_t *e, lepic_species_mixed_t *m, const lepic_phys_t &P,

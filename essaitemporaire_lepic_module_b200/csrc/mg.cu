@@ -601,8 +601,7 @@ struct SPArgs {
   int *out_i;
   double *out_d;
   double *host;               // pinned host memory for k, status, ktot, res (or null)
-  unsigned *barrier;          // this launch's barrier word, the device error word
-  int *err;
+  GridBarrier barrier;
 };
 
 extern __shared__ __align__(16) unsigned char sp_smem[];
@@ -692,7 +691,12 @@ __device__ __forceinline__ double smooth(const SPArgs &a, int level, int &cur, b
       if (dig == 0) {
         res = total<GRID>(l & 1, sh, a.partial);
         stopped = res <= eps_abs;
-        if (!GRID && l % SWEEPS_PER_BEAT == 0) grid.beat();
+        if (l % SWEEPS_PER_BEAT == 0) {
+          if (!GRID)
+            grid.beat();
+          else if (grid.dead())
+            stopped = true;
+        }
       } else if (l >= 3) {
         const double before = l == 3 ? total<GRID>((l - 1) & 1, sh, a.partial) : res;
         res = total<GRID>(l & 1, sh, a.partial);
@@ -843,7 +847,7 @@ __device__ __noinline__ void split_out(const SPArgs &a, int cur) {
 template <class Sync>
 __global__ void __launch_bounds__(SP_BLOCK, 1) k_pdesolver_split(const __grid_constant__ SPArgs a) {
   using namespace mgs;
-  Sync grid(a.barrier, a.err);
+  Sync grid(a.barrier);
   __shared__ double sh[64];
   const int ng = a.ng, ls = a.ls, down = ls < ng ? ls : ng - 1;   // down: the last grid level restricted from
   unsigned curs = 0;   // bit l: the current red buffer of grid level l
@@ -873,7 +877,7 @@ __global__ void __launch_bounds__(SP_BLOCK, 1) k_pdesolver_split(const __grid_co
   double res_s = 0.0, ktot = 0.0, r = 0.0;
   int status = 0, k = 1;
   bool converged = false;
-  while (!converged) {
+  while (!converged && !grid.dead()) {
     const bool first = k == 1;
     int iter[MG_MAX + 1];
     for (int i = 0; i <= MG_MAX; ++i) iter[i] = 0;
@@ -882,7 +886,7 @@ __global__ void __launch_bounds__(SP_BLOCK, 1) k_pdesolver_split(const __grid_co
     const int mid = down + 1;
     for (int g = 1; g <= 2 * down + 1; ++g) {
       if (g == mid && ls < ng) {
-        if (blockIdx.x == 0) chip_cycle(a, first, iter, grid, sh);
+        if (blockIdx.x == 0 && !grid.dead()) chip_cycle(a, first, iter, grid, sh);
         grid.sync();
         continue;
       }
@@ -915,7 +919,7 @@ __global__ void __launch_bounds__(SP_BLOCK, 1) k_pdesolver_split(const __grid_co
       for (int i = 1; i <= ng; ++i) a.out_i[2 + i] = iter[i];
     k = k + 1;
   }
-  split_out(a, (curs >> 1) & 1);
+  if (!grid.dead()) split_out(a, (curs >> 1) & 1);
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     a.out_i[0] = k;
     a.out_i[1] = status;
@@ -928,6 +932,7 @@ __global__ void __launch_bounds__(SP_BLOCK, 1) k_pdesolver_split(const __grid_co
       a.host[3] = r;
     }
   }
+  grid.leave(a.out_i + 1, a.host ? a.host + 1 : nullptr);
 }
 
 // the solve's results to the host: waits for the stream, returns the status
@@ -949,7 +954,7 @@ int solve_results(const int *out_i, const double *out_d, int *k_out, double *kto
 // coefficients out of div_by's range): the caller takes the general kernel.
 int launch_split(const int n[3], const double h[3], double *u, const double *b, const int *bcnd, int ncycl,
                  double eps, double omega, int ng, double eps0, int *out_i, double *out_d, double *host,
-                 cudaStream_t s, bool &launched) {
+                 cudaStream_t s, bool &launched, unsigned rounds) {
   using Lev = mgs::Lev<double>;
   launched = false;
   if (Lev::elements(n[0], n[1], n[2]) >= 2130000000LL) return LEPIC_OK;
@@ -965,9 +970,8 @@ int launch_split(const int n[3], const double h[3], double *u, const double *b, 
   A.out_i = out_i;
   A.out_d = out_d;
   A.host = host;
-  A.barrier = grid_barrier();
-  A.err = ctx().d_err;
-  if (!A.barrier) return LEPIC_ERR_CUDA;
+  A.barrier = grid_barrier(rounds);
+  if (!A.barrier.line) return LEPIC_ERR_CUDA;
   for (int l = 1; l <= ng; ++l) {
     Lev &L = A.L[l];
     L.shape(n[0] >> (l - 1), n[1] >> (l - 1), n[2] >> (l - 1));
@@ -1035,7 +1039,7 @@ int launch_split(const int n[3], const double h[3], double *u, const double *b, 
 
 int launch_pdesolver(const Dims &d, const double h[3], double *u, const double *b, const int *bcnd,
                      int ncycl, double eps, double omega, int ng, double eps0, int *k_out,
-                     double *ktot_out, double *res_out, cudaStream_t s, int pbc, int nmn) {
+                     double *ktot_out, double *res_out, cudaStream_t s, int pbc, int nmn, unsigned rounds) {
   if (ng < 1 || ng > MG_MAX) return LEPIC_ERR_ARG;
   const bool gen = pbc || nmn;
   int n[3] = {d.n1, d.n2, d.n3};
@@ -1048,7 +1052,7 @@ int launch_pdesolver(const Dims &d, const double h[3], double *u, const double *
   bool launched = false;
   double *host = gen ? nullptr : result_block();
   if (!gen)
-    if (int rc = launch_split(n, h, u, b, bcnd, ncycl, eps, omega, ng, eps0, out_i, out_d, host, s, launched))
+    if (int rc = launch_split(n, h, u, b, bcnd, ncycl, eps, omega, ng, eps0, out_i, out_d, host, s, launched, rounds))
       return rc;
   if (launched && host) {
     LEPIC_CUDA(cudaStreamSynchronize(s));

@@ -75,8 +75,7 @@ struct XArgs {
   int *out_i;      // [0] refinement iterations, [1] status
   double *out_d;   // [0] res/alpha, [1] first res/alpha
   double *host;    // pinned host memory for refinements, status, res/alpha (or null)
-  unsigned *barrier;   // this launch's barrier word, the device error word
-  int *err;
+  GridBarrier barrier;
 };
 
 extern __shared__ __align__(16) unsigned char xm_smem[];
@@ -221,7 +220,12 @@ __device__ __forceinline__ void sweeps(const XArgs &a, const Lev &L, int nu, boo
   const float om = a.omega;
   for (int s = 0; s < nu; ++s) {
     const bool last = s == nu - 1, add = GRID && addu && last;
-    if (!GRID && s % SWEEPS_PER_BEAT == SWEEPS_PER_BEAT - 1) grid.beat();
+    if (s % SWEEPS_PER_BEAT == SWEEPS_PER_BEAT - 1) {
+      if (!GRID)
+        grid.beat();
+      else if (grid.dead())
+        break;
+    }
     if (s > 0 || !started) {
       if (add)
         colour_phase<float, XV, mgs::RED, DO_RELAX | DO_ADDU, !GRID>(L, L.red[0], L.red[0], L.black, om, w, nullptr,
@@ -329,7 +333,7 @@ __device__ __noinline__ void add_u(const XArgs &a) {
 
 template <class Sync, int BLOCK>
 __global__ void __launch_bounds__(BLOCK, 1) k_refine_mixed(const __grid_constant__ XArgs a) {
-  Sync grid(a.barrier, a.err);
+  Sync grid(a.barrier);
   __shared__ double sh[32];
   const int ng = a.ng, ls = a.ls, down = ls < ng ? ls : ng - 1;   // down: the last grid level restricted from
   {
@@ -370,7 +374,7 @@ __global__ void __launch_bounds__(BLOCK, 1) k_refine_mixed(const __grid_constant
     acc += residual_f64<BLACK>(a, L1, start1, mgs::grid_team());
     res = grid_sum(a, acc, it, grid, sh) / a.alpha;
     if (res0 < 0.0) res0 = res;
-    if (res < a.eps) break;
+    if (grid.dead() || res < a.eps) break;
     if (it >= a.max_refine) {
       status = LEPIC_ERR_NOT_CONVERGED;
       break;
@@ -386,7 +390,7 @@ __global__ void __launch_bounds__(BLOCK, 1) k_refine_mixed(const __grid_constant
     bool added = false;
     for (int g = 1; g <= 2 * down + 1; ++g) {
       if (g == mid && ls < ng) {
-        if (blockIdx.x == 0) chip_cycle(a, first, grid);
+        if (blockIdx.x == 0 && !grid.dead()) chip_cycle(a, first, grid);
         grid.sync();
         continue;
       }
@@ -410,7 +414,7 @@ __global__ void __launch_bounds__(BLOCK, 1) k_refine_mixed(const __grid_constant
     }
     ++it;
   }
-  split_out(a);
+  if (!grid.dead()) split_out(a);
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     a.out_i[0] = it;
     a.out_i[1] = status;
@@ -422,6 +426,7 @@ __global__ void __launch_bounds__(BLOCK, 1) k_refine_mixed(const __grid_constant
       a.host[2] = res;
     }
   }
+  grid.leave(a.out_i + 1, a.host ? a.host + 1 : nullptr);
 }
 
 }  // namespace
@@ -435,7 +440,7 @@ __global__ void k_solve_status(const int *out_i, int *err) {
 int launch_pdesolver_mixed(const Dims &d, const double h[3], double *u, const double *b, const int *bcnd,
                            double eps, double omega, int ng, double eps0, int max_refine, int nu_fine_pre,
                            int nu_fine_post, int nu_pre, int nu_post, int coarse_sweeps, int *iters,
-                           double *res_out, cudaStream_t s) {
+                           double *res_out, cudaStream_t s, unsigned rounds) {
   if (ng < 1 || ng > XM_MAX) return LEPIC_ERR_ARG;
   const int n[3] = {d.n1, d.n2, d.n3};
   for (int q = 0; q < 3; ++q)
@@ -455,9 +460,8 @@ int launch_pdesolver_mixed(const Dims &d, const double h[3], double *u, const do
   A.b = b;
   A.bcnd = bcnd;
   A.eps = eps;
-  A.barrier = grid_barrier();
-  A.err = c.d_err;
-  if (!A.barrier) return LEPIC_ERR_CUDA;
+  A.barrier = grid_barrier(rounds);
+  if (!A.barrier.line) return LEPIC_ERR_CUDA;
   if (Lev::elements(n[0], n[1], n[2]) >= 2130000000LL) return LEPIC_ERR_UNSUPPORTED;   // 32-bit element numbers
   // shapes and coefficients per level (Src/mg.h)
   for (int l = 1; l <= ng; ++l) {

@@ -90,28 +90,32 @@ struct Lev {
 // (0.3 us by itself, the cooperative groups' barrier of the grid 1.2).
 // The grid's barrier is a word of its own per launch (grid_barrier()): each
 // block adds 1, block 0 what takes the word to its top bit flipped and the
-// count back to where it was, and the blocks watch that bit.  Unlike the
-// cooperative groups' barrier nothing waits for the addition's result, and the
-// read that sees the bit is the acquire (with relaxed reads and a fence behind
-// them the mixed solve of 48x40x56 took 468 us instead of 421).  Solves at
-// 128^3: FP64 4.32 -> 4.07 ms, mixed 613 -> 582 us; at 256^3 mixed 12.4 -> 11.2
-// ms.  The blocks are co-resident (cooperative launch) and a phase takes
+// count back to 0, and the blocks watch that bit.  Unlike the cooperative
+// groups' barrier nothing waits for the addition's result, and the read that
+// sees the bit is the acquire (with relaxed reads and a fence behind them the
+// mixed solve of 48x40x56 took 468 us instead of 421).  Solves at 128^3: FP64
+// 4.32 -> 4.07 ms, mixed 613 -> 582 us; at 256^3 mixed 12.4 -> 11.2 ms.
+//
+// The blocks are co-resident (cooperative launch) and a phase takes
 // milliseconds at most, but for block 0's on the levels on chip, which may
 // smooth the coarsest one a million times: it counts its sweeps there in a
 // second word (beat).  A wait therefore lasts as long as anything moves,
 // arrivals or beats; where nothing has for BARRIER_ROUNDS rounds of looks (one
-// and a half seconds; counted in looks, since a process that shares the
-// device may stop this one for any time), the block records LEPIC_ERR_TIMEOUT
-// and waits no more.
-constexpr unsigned BARRIER_LOOKS = 1u << 12, BARRIER_ROUNDS = 1u << 10;
+// and a half seconds; counted in looks, since a process that shares the device
+// may stop this one for any time), the block gives up: it neither arrives nor
+// waits at any barrier any more, ends its cycle on what the level arrays hold
+// and leaves phi alone; the others no longer get past a barrier and do the
+// same.  The last block to leave then clears the word, whose count the missing
+// arrivals have left anywhere, for the launch that has it next, and makes
+// LEPIC_ERR_TIMEOUT the solve's status.
+constexpr unsigned BARRIER_LOOKS = 1u << 12;
 constexpr int SWEEPS_PER_BEAT = 256;
 struct GridSync {
-  enum { WORD = 0, BEAT = 1 };   // of the launch's line
+  enum { WORD = 0, BEAT = 1, LEFT = 2, SPARE = 4 };   // of the launch's line
   struct State {
     unsigned *line, phase;
-    int *err;
     bool dead;
-    unsigned moved, idle;   // what had moved after the last round, rounds without any since
+    unsigned rounds, moved, idle;   // the limit; what had moved after the last round, rounds without any since
   };
   static __device__ __forceinline__ State &state() {
     __shared__ State s;
@@ -123,8 +127,8 @@ struct GridSync {
     return v;
   }
   // (the bit cannot flip before this block has arrived once)
-  __device__ GridSync(unsigned *line, int *err) {
-    if (threadIdx.x == 0) state() = {line, look(line + WORD) & 0x80000000u, err, false, 0, 0};
+  __device__ explicit GridSync(const GridBarrier &g) {
+    if (threadIdx.x == 0) state() = {g.line, look(g.line + WORD) & 0x80000000u, false, g.rounds, 0, 0};
   }
   // looks at `word` until its top bit differs from phase's, BARRIER_LOOKS
   // times at most: what is left of them (a loop of its own instructions: with
@@ -146,9 +150,9 @@ struct GridSync {
     const unsigned moved = look(s.line + WORD) + look(s.line + BEAT);
     s.idle = moved != s.moved ? 0 : s.idle + 1;
     s.moved = moved;
-    if (s.idle < BARRIER_ROUNDS) return false;
+    if (s.idle < s.rounds) return false;
     s.dead = true;
-    raise_err(s.err, LEPIC_ERR_TIMEOUT, (int)blockIdx.x);
+    s.line += SPARE;   // its arrivals go there from now on (a test before each would delay the living ones')
     return true;
   }
   __device__ __forceinline__ void sync() {
@@ -164,13 +168,36 @@ struct GridSync {
     }
     __syncthreads();
   }
+  // this block has given up (the same for all of its threads between barriers)
+  __device__ __forceinline__ bool dead() const { return state().dead; }
+  // the end of the kernel: every block calls it once.  status, host: where
+  // block 0 has put the solve's status (host may be null).
+  __device__ __forceinline__ void leave(int *status, double *host) {
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    const State &s = state();
+    const unsigned mine = s.dead ? 0x10001u : 1u;   // the blocks that left, and of them those that had given up
+    __threadfence();
+    unsigned *const line = s.dead ? s.line - SPARE : s.line;
+    const unsigned left = atomicAdd(line + LEFT, mine) + mine;
+    if ((left & 0xffffu) != gridDim.x) return;
+    __threadfence();
+    line[LEFT] = 0;
+    if (left >> 16) {
+      line[WORD] = 0;
+      *status = LEPIC_ERR_TIMEOUT;
+      if (host) *host = LEPIC_ERR_TIMEOUT;
+    }
+  }
   // block 0 on the levels on chip: the others' wait goes on
   __device__ __forceinline__ void beat() {
     if (threadIdx.x == 0) asm volatile("red.relaxed.gpu.global.add.u32 [%0], 1;" ::"l"(state().line + BEAT));
   }
 };
 struct ClusterSync {
-  __device__ ClusterSync(unsigned *, int *) {}
+  __device__ explicit ClusterSync(const GridBarrier &) {}
+  __device__ __forceinline__ bool dead() const { return false; }
+  __device__ __forceinline__ void leave(int *, double *) {}
   __device__ __forceinline__ void beat() {}
   __device__ __forceinline__ void sync() {
     asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");

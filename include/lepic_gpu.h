@@ -787,6 +787,17 @@ int lepic_dev_check_async(void *stream, int *host);
  * launch status; the recorded one is read with lepic_dev_check.  No
  * counterpart in the reference. */
 int lepic_dev_wait_selftest(long long limit_ns, void *stream);
+/* The failure path of a Poisson solve whose barrier between its blocks is
+ * given up, for tests: one cycle of lepic_dev_pdesolver with eps = 0, or
+ * (mixed) one refinement of lepic_dev_pdesolver_mixed with 20,000 sweeps of the
+ * coarsest level, by blocks that wait a few milliseconds at most, so that on a
+ * grid solved by the whole device (above 60,000 elements per colour, 50^3)
+ * whose coarsest level is smoothed by one block they give up meanwhile.
+ * Returns LEPIC_ERR_TIMEOUT, or without wait (mixed only) the launch status,
+ * with LEPIC_ERR_TIMEOUT in the device error word; u is undefined then.  No
+ * counterpart in the reference. */
+int lepic_dev_solve_selftest(const lepic_grid_t *g, double *u, const double *b, int ng, const lepic_phys_t *P,
+                             int mixed, int wait, void *stream);
 /* Library build identification (nvcc version, arch). */
 const char *lepic_build_info(void);
 

@@ -8,6 +8,8 @@ context stays usable afterwards.
   * a refinement cap too small for the tolerance  -> LEPIC_ERR_NOT_CONVERGED (23)
   * a NaN in the right-hand side                  -> a non-zero status, then a
                                                      clean solve succeeds
+  * a solve whose barrier is given up             -> LEPIC_ERR_TIMEOUT (25),
+                                                     then solves are right
   * a bounded device wait that nothing completes  -> LEPIC_ERR_TIMEOUT (25)
                                                      after its limit, then the
                                                      context runs a step
@@ -115,6 +117,63 @@ def test_bounded_wait_times_out_and_context_stays_usable():
     sim.step()
     torch.cuda.synchronize()
     assert L.lepic_dev_check(None, C.byref(detail)) == 0
+
+
+@pytest.mark.parametrize("how", ["f64", "mixed", "mixed_nonblocking"])
+def test_a_solve_whose_barrier_is_given_up_says_so(how):
+    """Blocks that wait a few milliseconds only, while block 0 smooths the
+    coarsest level for longer: the solve ends with LEPIC_ERR_TIMEOUT (without
+    a wait, in the error word, read here without clearing anything else), and
+    the next 70 solves, which come round to the same barrier, are those of
+    before."""
+    import ctypes as C
+
+    import torch
+    from essaitemporaire_lepic_module_b200._lib import LepicGrid, lib, phys_struct
+    L = lib()
+    st = config.build("box16")
+    mixed = how != "f64"
+    n, ng = (64, 64, 64), 3 if mixed else 4
+    shape = tuple(v + 3 for v in n)
+    bc = np.ones(shape, dtype=np.int32)
+    bc[2:-2, 2:-2, 2:-2] = -1
+    bct = torch.as_tensor(bc, device="cuda")
+    rt = torch.as_tensor(np.random.default_rng(3).normal(size=tuple(v - 1 for v in shape)) * 1e-5, device="cuda")
+    grid = LepicGrid()
+    for a in range(3):
+        grid.n[a], grid.h[a] = n[a], 1.0e-4
+    grid.bcnd = bct.data_ptr()
+    P = phys_struct(st)
+    s = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+
+    def solve(entry):
+        u = torch.zeros(shape, dtype=torch.float64, device="cuda")
+        k, kt, res = C.c_int(0), C.c_double(0), C.c_double(0)
+        if entry == "f64":
+            rc = L.lepic_dev_pdesolver(C.byref(grid), C.c_void_p(u.data_ptr()), C.c_void_p(rt.data_ptr()), 1, 1e-9,
+                                       1.4, 4, C.byref(P), C.byref(k), C.byref(kt), C.byref(res), s)
+        else:
+            rc = L.lepic_dev_pdesolver_mixed(C.byref(grid), C.c_void_p(u.data_ptr()), C.c_void_p(rt.data_ptr()), 1e-9,
+                                             1.3, 4, C.byref(P), 40, 1, 3, 2, 2, 4, C.byref(k), C.byref(res), s)
+        assert rc == 0, (entry, rc)
+        return u
+
+    before = {e: solve(e) for e in ("f64", "mixed")}
+    u = torch.zeros(shape, dtype=torch.float64, device="cuda")
+    rc = L.lepic_dev_solve_selftest(C.byref(grid), C.c_void_p(u.data_ptr()), C.c_void_p(rt.data_ptr()), ng,
+                                    C.byref(P), int(mixed), int(how == "mixed"), s)
+    word = torch.zeros(2, dtype=torch.int32).pin_memory()
+    if how == "mixed_nonblocking":
+        assert rc == 0
+        assert L.lepic_dev_check_async(s, C.c_void_p(word.data_ptr())) == 0
+        torch.cuda.synchronize()
+        assert int(word[0]) == 25
+    else:
+        assert rc == 25
+        assert L.lepic_dev_check(s, None) == 0
+    for i in range(70):
+        e = ("f64", "mixed")[i % 2]
+        assert bool((solve(e) == before[e]).all())
 
 
 def test_nonblocking_loop_reports_failures_later():
