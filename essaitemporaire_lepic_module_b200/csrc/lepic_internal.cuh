@@ -544,24 +544,8 @@ __device__ __forceinline__ double quot(double a, double b, double y) {
   return fabs(a) < 1e200 ? div_by(a, b, y) : a * y;
 }
 
-// ------------------------------------------------ async copies and mbarriers
+// ------------------------------------------------------------ async copies
 __device__ __forceinline__ uint32_t smem_addr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ unsigned long long gtime() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-
-__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
 
 // a float4 from shared memory at 32-bit shared address a (a box staged
 // before a barrier and not written afterwards)
@@ -579,16 +563,6 @@ __device__ __forceinline__ void cp_async16(void *dst, const void *src) {
 __device__ __forceinline__ void cp_async4(void *dst, const void *src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
 }
-
-// wait for phase `parity` of the mbarrier, at most limit_ns of %globaltimer
-__device__ inline bool mbar_wait_ns(uint32_t bar, uint32_t parity, unsigned long long limit_ns) {
-  if (mbar_try(bar, parity)) return true;
-  const unsigned long long t0 = gtime();
-  while (!mbar_try(bar, parity))
-    if (gtime() - t0 > limit_ns) return false;
-  return true;
-}
-
 
 }  // namespace lepic
 

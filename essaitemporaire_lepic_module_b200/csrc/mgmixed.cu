@@ -437,6 +437,16 @@ __global__ void k_solve_status(const int *out_i, int *err) {
   if (out_i[1] != 0) raise_err(err, out_i[1], out_i[0]);
 }
 
+// The barrier's give-up by itself: two blocks, of which one waits for the
+// other, which leaves without having arrived.
+__global__ void k_wait_selftest(GridBarrier barrier, int *out_i) {
+  mgs::GridSync grid(barrier);
+  __syncthreads();
+  if (blockIdx.x == 0) grid.sync();
+  grid.leave(out_i + 1, nullptr);
+}
+constexpr long long ROUND_NS = 900000;   // a round of looks takes 0.95 ms
+
 int launch_pdesolver_mixed(const Dims &d, const double h[3], double *u, const double *b, const int *bcnd,
                            double eps, double omega, int ng, double eps0, int max_refine, int nu_fine_pre,
                            int nu_fine_post, int nu_pre, int nu_post, int coarse_sweeps, int *iters,
@@ -575,6 +585,19 @@ int pdesolver_mixed_stats(int *iters, double *res, cudaStream_t s) {
 }
 
 }  // namespace lepic
+
+extern "C" int lepic_dev_wait_selftest(long long limit_ns, void *stream) {
+  if (limit_ns <= 0 || limit_ns > 2000000000LL) return LEPIC_ERR_ARG;
+  const cudaStream_t s = (cudaStream_t)stream;
+  const lepic::GridBarrier barrier = lepic::grid_barrier((unsigned)((limit_ns + lepic::ROUND_NS - 1) / lepic::ROUND_NS));
+  int *out_i = (int *)lepic::scratch("wait_out_i", sizeof(int) * 2);
+  if (!barrier.line || !out_i) return LEPIC_ERR_CUDA;
+  LEPIC_CUDA(cudaMemsetAsync(out_i, 0, sizeof(int) * 2, s));
+  lepic::k_wait_selftest<<<2, 32, 0, s>>>(barrier, out_i);
+  lepic::k_solve_status<<<1, 1, 0, s>>>(out_i, lepic::ctx().d_err);
+  LEPIC_CUDA(cudaGetLastError());
+  return LEPIC_OK;
+}
 
 extern "C" int lepic_dev_pdesolver_mixed_stats(int *iters, double *res, void *stream) {
   return lepic::pdesolver_mixed_stats(iters, res, (cudaStream_t)stream);

@@ -100,9 +100,9 @@ struct Lev {
 // milliseconds at most, but for block 0's on the levels on chip, which may
 // smooth the coarsest one a million times: it counts its sweeps there in a
 // second word (beat).  A wait therefore lasts as long as anything moves,
-// arrivals or beats; where nothing has for BARRIER_ROUNDS rounds of looks (one
-// and a half seconds; counted in looks, since a process that shares the device
-// may stop this one for any time), the block gives up: it neither arrives nor
+// arrivals or beats; where nothing has for BARRIER_ROUNDS rounds of looks (about
+// a second; counted in looks, since a process that shares the device may stop
+// this one for any time), the block gives up: it neither arrives nor
 // waits at any barrier any more, ends its cycle on what the level arrays hold
 // and leaves phi alone; the others no longer get past a barrier and do the
 // same.  The last block to leave then clears the word, whose count the missing

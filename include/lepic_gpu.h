@@ -780,12 +780,13 @@ int lepic_dev_check(void *stream, int *detail);
  * or two later without stalling its launches.  Statuses recorded by kernels
  * on other streams between the copy and the clear are lost. */
 int lepic_dev_check_async(void *stream, int *host);
-/* The failure path of the bounded device waits, for tests: one block whose
- * first thread waits on an mbarrier phase that nothing completes, at most
- * limit_ns (0 < limit_ns <= 2e9) nanoseconds of %globaltimer, then records
- * LEPIC_ERR_TIMEOUT in the device error word; the context stays usable.  Returns the
- * launch status; the recorded one is read with lepic_dev_check.  No
- * counterpart in the reference. */
+/* The failure path of the bounded device waits (those of the Poisson solves'
+ * barrier between their blocks), for tests: a block waits at that barrier for
+ * another, which never arrives, for limit_ns (0 < limit_ns <= 2e9) nanoseconds,
+ * counted in looks at the barrier (rounded up to about a millisecond), then
+ * LEPIC_ERR_TIMEOUT is recorded in the device error word; the context stays
+ * usable.  Returns the launch status; the recorded one is read with
+ * lepic_dev_check.  No counterpart in the reference. */
 int lepic_dev_wait_selftest(long long limit_ns, void *stream);
 /* The failure path of a Poisson solve whose barrier between its blocks is
  * given up, for tests: one cycle of lepic_dev_pdesolver with eps = 0, or

@@ -92,10 +92,10 @@ def test_nan_in_rhs_is_reported_and_the_next_solve_works():
 
 
 def test_bounded_wait_times_out_and_context_stays_usable():
-    """An mbarrier phase that no copy completes: the wait gives up after its
-    limit (50 ms here; the library's copy waits allow one second) and the
-    kernel records LEPIC_ERR_TIMEOUT instead of hanging; the status is read
-    once and cleared, and a step runs afterwards."""
+    """A barrier that one of two blocks never reaches: the wait gives up after
+    its limit (50 ms here; the solves' allow about a second in which nothing
+    moves) and LEPIC_ERR_TIMEOUT is recorded instead of a hang; the
+    status is read once and cleared, and a step runs afterwards."""
     import ctypes as C
     import time
     import torch
