@@ -471,7 +471,7 @@ __device__ __forceinline__ void finish_push(int *count, int *side, double *acc, 
   for (int q = threadIdx.x >> 5; q < n; q += (int)(blockDim.x >> 5)) {
     double v = copies[lane * n + q] + copies[(lane + 32) * n + q];
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if (lane == 0 && v != 0.0) acc[q] += v;
+    if (lane == 0 && v != 0.0) atomicAdd(&acc[q], v);   // (another species' push may add to it on another stream)
   }
   if (threadIdx.x == 0) *count = *count - side[0];
 }

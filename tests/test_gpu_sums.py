@@ -123,3 +123,40 @@ def test_losses_are_all_counted(precision):
         assert pm[1, 0, p] == lost
         assert abs(pl[p, 0] - lost * ek) <= 1e-5 * lost * ek         # FP32 velocities in the mixed form
         assert abs(pm[1, 1, p] - pl[p, 0]) <= 1e-12 * pl[p, 0]
+
+
+@pytest.mark.parametrize("precision", ["f64", "mixed"])
+def test_losses_of_pushes_on_two_streams_share_an_array(precision):
+    """Two species pushed on two streams at once, their losses added to one
+    array: every lost particle of both is counted in it."""
+    import ctypes as C
+
+    import torch
+    from essaitemporaire_lepic_module_b200._lib import lib
+    from essaitemporaire_lepic_module_b200.sim import Simulation
+    st = _setup((16, 16, 16))
+    count = 4000
+    v = _place(st, count, "any")
+    v[:, :, 3] = 6e6 * np.where(np.arange(count) % 2, 1.0, -1.0)
+    sim = Simulation(st, cap=count + 37, precision=precision)
+    sim.load_from_host(v, [count] * st.ntype)
+    sim.sort()
+    sim.move_deposit()                           # the first call allocates
+    acc = torch.zeros(2 + 2 * (st.geom.ngrid + 1), dtype=torch.float64, device="cuda")
+    push = lib().lepic_dev_push_deposit_mixed if precision == "mixed" else lib().lepic_dev_push_deposit
+    E = sim.E32 if precision == "mixed" else sim.Ei
+    streams = [torch.cuda.Stream() for _ in sim.sp]
+    lost = 0
+    for _ in range(40):
+        sim.load_from_host(v, [count] * st.ntype)
+        sim.sort()
+        torch.cuda.synchronize()
+        for p, s in enumerate(sim.sp):
+            assert push(C.byref(sim.grid), C.c_void_p(E.data_ptr()), C.byref(s.s), p + 1, st.geom.ngrid,
+                        C.byref(sim.P), C.c_void_p(sim.np[p].data_ptr()), C.c_void_p(acc.data_ptr()), -1,
+                        C.c_void_p(streams[p].cuda_stream)) == 0
+        torch.cuda.synchronize()
+        lost += sum(count - s.n() for s in sim.sp)
+    sim.check_device()
+    assert lost > 1000
+    assert float(acc[2::2].sum()) == lost
