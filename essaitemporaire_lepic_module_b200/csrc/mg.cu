@@ -586,7 +586,7 @@ __global__ void __launch_bounds__(MG_BLOCK) k_pdesolver(const MGArgs *__restrict
 // 512 threads: with 768 and 1024 the phases spill (128^3: 4.8 and 5.8 ms).
 constexpr int SP_BLOCK = 512;
 constexpr long long SP_SMALL = 40000;   // elements per colour one cluster solves faster than the grid
-constexpr size_t SP_CHIP = 227000;   // shared memory of the levels on chip: 16^3 and below
+static_assert(MG_MAX == mgs::LEVELS, "the shared memory of their descriptors");
 
 struct SPArgs {
   mgs::Lev<double> L[MG_MAX + 2];   // levels 1..ng; after them level ls + 1 with its arrays on the grid
@@ -990,7 +990,7 @@ int launch_split(const int n[3], const double h[3], double *u, const double *b, 
   A.ls = ng;
   for (int l = ng; l >= 2; --l) {
     const size_t need = ((size_t)A.L[l].len * (8 * (l == ng ? 5 : 6) + 1) + 15) & ~(size_t)15;
-    if (csm + need > SP_CHIP) break;
+    if (csm + need > mgs::CHIP) break;
     A.oc[l] = (unsigned)csm;
     csm += need;
     A.ls = l - 1;

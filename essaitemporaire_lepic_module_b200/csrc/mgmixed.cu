@@ -47,7 +47,7 @@ using mgs::RED;
 using mgs::Team;
 using Lev = mgs::Lev<float>;
 
-constexpr int XM_MAX = 13;      // multigrid levels
+constexpr int XM_MAX = mgs::LEVELS;   // multigrid levels
 // threads per block: twice as many, at half the registers, on grids whose
 // finest level moves through HBM (a solve, with the cooperative groups'
 // barrier: 256^3 13.9 -> 12.7 ms, 192^3 and 176^3 the same, 160^3 10.4 -> 11.3
@@ -56,7 +56,6 @@ constexpr int XM_BLOCK = 512, XM_BLOCK_LARGE = 1024;
 constexpr long long XM_LARGE = 3000000;   // elements per colour from which it takes those
 constexpr int XV = 4;           // elements per 16-byte load
 constexpr long long XM_SMALL = 60000;  // elements per colour one cluster solves faster than the grid
-constexpr size_t XM_CHIP = 227000;   // shared memory of the levels on chip
 
 struct XArgs {
   Lev L[XM_MAX + 2];          // levels 1..ng; after them level ls + 1 with its arrays on the grid
@@ -500,7 +499,7 @@ int launch_pdesolver_mixed(const Dims &d, const double h[3], double *u, const do
   A.ls = ng;
   for (int l = ng; l >= 2; --l) {
     const size_t need = ((size_t)A.L[l].len * (4 * (l < ng ? 6 : 4) + 1) + 15) & ~(size_t)15;
-    if (csm + need > XM_CHIP) break;
+    if (csm + need > mgs::CHIP) break;
     A.oc[l] = (unsigned)csm;
     csm += need;
     A.ls = l - 1;

@@ -526,13 +526,20 @@ __device__ __forceinline__ void prolong_to(const Lev<T> &F, const Lev<T> &C, T *
 
 // Launch of a solve: `one` (its ClusterSync instance) as one cluster when the
 // finest level has at most `small` elements per colour and such a cluster
-// fits the device, else `all` (GridSync) cooperatively on every SM.
+// fits the device, else `all` (GridSync) cooperatively on every SM.  A
+// kernel's limit on dynamic shared memory is the same at every launch, the most
+// one takes: with each launch's own, two threads that solve on different grids
+// lower each other's between setting it and the launch.
+constexpr size_t CHIP = 227000;   // for the levels on chip: 16^3 and below
+constexpr int LEVELS = 13;        // multigrid levels at most
+constexpr size_t SMEM_MOST = CHIP + sizeof(Lev<double>) * (LEVELS + 1);
+static_assert(SMEM_MOST + 2048 <= 232448, "beside the kernels' static shared memory");
 inline cudaError_t launch_solve(const void *all, const void *one, void **args, long long elements, long long small,
                                 int threads, size_t smem, int sms, cudaStream_t s) {
   cudaError_t e = cudaSuccess;
   if (elements <= small) {
     e = cudaFuncSetAttribute(one, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(one, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(one, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MOST);
     if (e != cudaSuccess) return e;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
@@ -549,7 +556,7 @@ inline cudaError_t launch_solve(const void *all, const void *one, void **args, l
     if (cudaOccupancyMaxActiveClusters(&n, one, &c) == cudaSuccess && n >= 1) return cudaLaunchKernelExC(&c, one, args);
     cudaGetLastError();
   }
-  e = cudaFuncSetAttribute(all, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  e = cudaFuncSetAttribute(all, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MOST);
   if (e != cudaSuccess) return e;
   return cudaLaunchCooperativeKernel(all, dim3(sms), dim3(threads), args, smem, s);
 }

@@ -156,3 +156,65 @@ def test_the_grid_waits_for_a_million_sweeps_on_chip():
     assert float((phis[0] - phis[1]).abs().max()) <= 1e-5 * float(phis[0].abs().max())
     detail = C.c_int(0)
     assert L.lepic_dev_check(s, C.byref(detail)) == 0
+
+
+@pytest.mark.parametrize("mixed", [False, True])
+def test_solves_of_several_threads(mixed):
+    """Six host threads solving on grids of two sizes, on one stream (FP64:
+    each waits for its own solve): every solve succeeds and is the one its
+    thread gets alone."""
+    import threading
+
+    import torch
+    from essaitemporaire_lepic_module_b200 import config
+    from essaitemporaire_lepic_module_b200._lib import LepicGrid, lib, phys_struct
+
+    P = phys_struct(config.build("box16"))
+    s = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+
+    def case(n, ng):
+        shape = tuple(v + 3 for v in reversed(n))
+        bc = np.ones(shape, dtype=np.int32)
+        bc[2:-2, 2:-2, 2:-2] = -1
+        bct = torch.as_tensor(bc, device="cuda")
+        rt = torch.as_tensor(np.random.default_rng(n[0]).normal(size=tuple(v - 1 for v in shape)) * 1e-5,
+                             device="cuda")
+        grid = LepicGrid()
+        for a in range(3):
+            grid.n[a], grid.h[a] = n[a], 1.0e-4
+        grid.bcnd = bct.data_ptr()
+        u = torch.zeros(shape, dtype=torch.float64, device="cuda")
+        torch.cuda.synchronize()
+
+        def run():
+            k, kt, res = C.c_int(0), C.c_double(0), C.c_double(0)
+            with torch.cuda.stream(torch.cuda.default_stream()):
+                u.zero_()
+            if mixed:
+                return lib().lepic_dev_pdesolver_mixed(
+                    C.byref(grid), C.c_void_p(u.data_ptr()), C.c_void_p(rt.data_ptr()), 1e-9, 1.3, ng, C.byref(P),
+                    60, 1, 3, 2, 2, 4, None, None, s)
+            return lib().lepic_dev_pdesolver(C.byref(grid), C.c_void_p(u.data_ptr()), C.c_void_p(rt.data_ptr()), 3,
+                                             1e-9, 1.4, ng, C.byref(P), C.byref(k), C.byref(kt), C.byref(res), s)
+        return run, u, (bct, rt)
+
+    # one kernel (a cluster); 16^3 and below on chip, nothing on chip
+    cases = [case((32, 32, 32), 4) if i % 2 else case((10, 14, 18), 1) for i in range(6)]
+    want = []
+    for run, u, _ in cases:
+        assert run() == 0
+        want.append(u.clone())
+    failed = []
+
+    def work(i):
+        run, u, _ = cases[i]
+        rcs = [run() for _ in range(300)]
+        if any(rcs) or not bool((u == want[i]).all()):
+            failed.append((i, [rc for rc in rcs if rc][:1]))
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(len(cases))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed
+    assert lib().lepic_dev_check(s, None) == 0
