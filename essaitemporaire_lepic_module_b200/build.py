@@ -39,7 +39,7 @@ def nvcc():
 
 def _deps():
     inc = os.path.join(os.path.dirname(HERE), "include", "lepic_gpu.h")
-    hdrs = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith(".cuh")] + [inc]
+    hdrs = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cuh", ".h"))] + [inc]
     return max(os.path.getmtime(h) for h in hdrs)
 
 

@@ -6,6 +6,7 @@
 #include <cstdio>
 
 #include "../../include/lepic_gpu.h"
+#include "poisson_scale.h"
 
 namespace lepic {
 

@@ -1021,7 +1021,7 @@ int launch_split(const int n[3], const double h[3], double *u, const double *b, 
     }
     L.m = reinterpret_cast<unsigned char *>(p + halves * n8);
   }
-  A.alpha = fabs((double)((n[0] + 1) * (n[1] + 1) * (n[2] + 1)) * A.L[1].ac) * 1.0;
+  A.alpha = residual_scale(n, A.L[1].ac);
   const int blocks = ctx().sms;
   A.partial = (double *)scratch("mgs_partial", sizeof(double) * 2 * blocks);
   if (!A.partial) return LEPIC_ERR_CUDA;
@@ -1117,7 +1117,7 @@ int launch_pdesolver(const Dims &d, const double h[3], double *u, const double *
     }
   }
   double ac = A.L[1].ac;
-  A.alpha = fabs((double)((n[0] + 1) * (n[1] + 1) * (n[2] + 1)) * ac) * 1.0;
+  A.alpha = residual_scale(n, ac);
   void *kern = gen ? (void *)k_pdesolver<true> : (void *)k_pdesolver<false>;
   int occ = 0;
   LEPIC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, MG_BLOCK, 0));
@@ -1264,7 +1264,7 @@ extern "C" int lepic_dev_pdesolver_noalloc(const lepic_grid_t *g, double *u, con
             n[0], n[1], n[2], ng, MG_NOALLOC_BYTES);
     return LEPIC_ERR_SCRATCH_LIMIT;
   }
-  A.alpha = fabs((double)((n[0] + 1) * (n[1] + 1) * (n[2] + 1)) * A.L[1].ac) * 1.0;
+  A.alpha = residual_scale(n, A.L[1].ac);
   // the shared array keeps the previous call's contents: clear the fine
   // residual arrays whose ghost entries the restriction may read
   for (int l = 1; l < ng; ++l) LEPIC_CUDA(cudaMemsetAsync(rf_ptr[l], 0, rf_bytes[l], s));

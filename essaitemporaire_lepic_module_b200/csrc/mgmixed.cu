@@ -535,7 +535,7 @@ int launch_pdesolver_mixed(const Dims &d, const double h[3], double *u, const do
       A.bs[q] = p + (2 + q) * len;
     }
   }
-  A.alpha = fabs((double)((n[0] + 1) * (n[1] + 1) * (n[2] + 1)) * A.ac) * 1.0;
+  A.alpha = residual_scale(n, A.ac);
   const int blocks = c.sms;
   A.partial = (double *)scratch("xm_partial", sizeof(double) * 2 * blocks);
   A.out_i = (int *)scratch("xm_out_i", sizeof(int) * 4);

@@ -136,3 +136,19 @@ def test_residency_switch_and_host_statements_without_mirrors():
     assert L.lepic_gpu_mirror_stats(C.byref(h2d), C.byref(d2h), C.byref(m)) == 0
     assert m.value == 0
     assert L.lepic_gpu_set_residency(0) == 0 and L.lepic_gpu_residency() == 0
+
+
+@pytest.mark.parametrize("n", [(16, 16, 16), (5, 9, 7), (1290, 1290, 1290), (1296, 1296, 1296), (1600, 1600, 1600)])
+def test_scale_of_the_poisson_residual(n, tmp_path):
+    """The number of nodes in it does not wrap (from 1290^3 on it is above
+    2^31, and 1600^3 above 2^32)."""
+    import subprocess
+    src = tmp_path / "scale.cpp"
+    src.write_text('#include <cstdio>\n#include "poisson_scale.h"\nint main() {\n'
+                   f'  const int n[3] = {{{n[0]}, {n[1]}, {n[2]}}};\n'
+                   '  std::printf("%.17g", lepic::residual_scale(n, -0.75));\n}\n')
+    exe = tmp_path / "scale"
+    subprocess.run(["g++", "-O2", "-I", os.path.join(ROOT, "essaitemporaire_lepic_module_b200", "csrc"), str(src), "-o",
+                    str(exe)], check=True)
+    got = float(subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout)
+    assert got == 0.75 * (n[0] + 1) * (n[1] + 1) * (n[2] + 1)
