@@ -2,8 +2,10 @@
 the general kernel (lepic_dev_pdesolver_noalloc runs it): the same node
 arithmetic in the same order, so phi, cycles and sweeps are compared bit for
 bit.  Grids at the edges of the split layout: odd and even row lengths, one
-level, levels on the grid and on chip; walls anywhere, free ghost nodes and
-labels 0 and -2 among them."""
+level, levels on the grid and on chip; solved by one cluster (up to 40,000
+elements per colour) and by the whole device, the coarsest level on chip and
+on the grid in both; walls anywhere, free ghost nodes and labels 0 and -2
+among them."""
 import ctypes as C
 
 import numpy as np
@@ -16,7 +18,9 @@ pytestmark = [pytest.mark.gpu,
 
 
 @pytest.mark.parametrize("n,ng", [((5, 9, 7), 1), ((6, 10, 14), 2), ((30, 22, 26), 2), ((16, 16, 16), 5),
-                                  ((32, 16, 24), 4), ((40, 24, 32), 4), ((66, 34, 18), 2), ((64, 64, 64), 7)])
+                                  ((32, 16, 24), 4), ((40, 24, 32), 4), ((66, 34, 18), 2), ((64, 64, 64), 7),
+                                  ((63, 55, 61), 1), ((64, 64, 64), 2), ((62, 58, 54), 2), ((60, 52, 64), 3),
+                                  ((40, 38, 38), 2)])
 @pytest.mark.parametrize("walls", ["box", "any"])
 def test_split_equals_general_kernel(n, ng, walls):
     import torch
@@ -61,13 +65,16 @@ def test_split_equals_general_kernel(n, ng, walls):
         assert np.array_equal(a[4], b[4])
 
 
-@pytest.mark.parametrize("n,ng", [((9, 7, 6), 1), ((10, 14, 18), 2), ((24, 32, 40), 4), ((72, 40, 56), 4)])
+@pytest.mark.parametrize("n,ng", [((9, 7, 6), 1), ((10, 14, 18), 2), ((24, 32, 40), 4), ((72, 40, 56), 4),
+                                  ((76, 52, 68), 3), ((184, 176, 200), 4)])
 @pytest.mark.parametrize("nu", [(1, 3, 2, 2, 4), (0, 3, 0, 2, 1), (2, 1, 1, 1, 8), (1, 0, 2, 0, 4)])
 def test_mixed_schedules_reach_the_fp64_solution(n, ng, nu):
     """FP32 cycles of any schedule (sweeps before and after on the finest and
     on the coarser levels, on the coarsest; 0 among them) in FP64 refinement:
     the same potential as the FP64 multigrid, both to a residual of 1e-11 of
-    the first one, from which phi is off by less than 1e-6."""
+    the first one, from which phi is off by less than 1e-6.  By one cluster,
+    by the whole device, and there (from 3e6 elements per colour) with 1024
+    threads per block."""
     import torch
     from essaitemporaire_lepic_module_b200 import config
     from essaitemporaire_lepic_module_b200._lib import LepicGrid, lib, phys_struct
