@@ -74,6 +74,17 @@ void *scratch(const char *name, size_t bytes) {
   return b.p;
 }
 
+void scratch_drop(const char *prefix) {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  std::lock_guard<std::mutex> lk(g_mu);
+  for (auto &kv : g_scratch) {
+    if (kv.first.first != dev || kv.first.second.compare(0, strlen(prefix), prefix) != 0) continue;
+    if (kv.second.p) cudaFree(kv.second.p);   // (waits for the kernels that use it)
+    kv.second = Buf{};
+  }
+}
+
 namespace {
 struct ResultBlock {
   double *p = nullptr;

@@ -46,6 +46,7 @@ struct Ctx {
 };
 Ctx &ctx();                                     // context of the current device
 void *scratch(const char *name, size_t bytes);  // cached device buffer (grows)
+void scratch_drop(const char *prefix);          // give back the buffers whose names begin so
 int check_err(cudaStream_t s);                  // sync, read + clear device error word
 // The calling thread's block of pinned host memory for the few results of a
 // kernel that it launches and waits for (the kernel writes them there, which

@@ -951,7 +951,9 @@ int solve_results(const int *out_i, const double *out_d, int *k_out, double *kto
 
 // The split solve's arrays and launch; LEPIC_OK with launched = false where it
 // does not apply (a level with too many nodes for its 32-bit element numbers,
-// coefficients out of div_by's range): the caller takes the general kernel.
+// coefficients out of div_by's range, no device memory for its copies: 32
+// bytes per grid node, against 12 of the general kernel): the caller takes the
+// general kernel.
 int launch_split(const int n[3], const double h[3], double *u, const double *b, const int *bcnd, int ncycl,
                  double eps, double omega, int ng, double eps0, int *out_i, double *out_d, double *host,
                  cudaStream_t s, bool &launched, unsigned rounds) {
@@ -1009,7 +1011,11 @@ int launch_split(const int n[3], const double h[3], double *u, const double *b, 
     char nm[32];
     snprintf(nm, sizeof nm, "mgs_%d", l);
     double *p = (double *)scratch(nm, (sizeof(double) * halves + 1) * n8);
-    if (!p) return LEPIC_ERR_CUDA;
+    if (!p) {
+      cudaGetLastError();
+      scratch_drop("mgs_");   // the general kernel may need what the other levels took
+      return LEPIC_OK;
+    }
     L.red[0] = p;
     L.red[1] = p + n8;
     L.black = p + 2 * n8;

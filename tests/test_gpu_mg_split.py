@@ -225,3 +225,43 @@ def test_solves_of_several_threads(mixed):
         t.join()
     assert not failed
     assert lib().lepic_dev_check(s, None) == 0
+
+
+def test_a_nearly_full_device_gets_the_general_kernel():
+    """Too little device memory for the split copies (32 bytes a node), enough
+    for the general kernel (12): the solve succeeds, with the same phi."""
+    import torch
+    from essaitemporaire_lepic_module_b200 import config
+    from essaitemporaire_lepic_module_b200._lib import LepicGrid, lib, phys_struct
+
+    P = phys_struct(config.build("box16"))
+    n, ng = (320, 320, 256), 6                    # 27e6 nodes: 0.97 and 0.36 GB with the buffers' margins
+    shape = tuple(v + 3 for v in reversed(n))
+    bct = torch.ones(shape, dtype=torch.int32, device="cuda")
+    bct[2:-2, 2:-2, 2:-2] = -1
+    g = torch.Generator(device="cuda").manual_seed(3)
+    rt = torch.randn(tuple(v - 1 for v in shape), dtype=torch.float64, device="cuda", generator=g) * 1e-5
+    grid = LepicGrid()
+    for a in range(3):
+        grid.n[a], grid.h[a] = n[a], 1.0e-4
+    grid.bcnd = bct.data_ptr()
+
+    def solve(u):
+        k, kt, res = C.c_int(0), C.c_double(0), C.c_double(0)
+        rc = lib().lepic_dev_pdesolver(C.byref(grid), C.c_void_p(u.data_ptr()), C.c_void_p(rt.data_ptr()), 2, 1e-9, 1.4,
+                                       ng, C.byref(P), C.byref(k), C.byref(kt), C.byref(res),
+                                       C.c_void_p(torch.cuda.current_stream().cuda_stream))
+        return rc, k.value, kt.value
+
+    u, w = torch.zeros(shape, dtype=torch.float64, device="cuda"), torch.zeros(shape, dtype=torch.float64, device="cuda")
+    eq = torch.empty(shape, dtype=torch.bool, device="cuda")
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    fill = torch.empty(torch.cuda.mem_get_info()[0] - 500 * 2 ** 20, dtype=torch.uint8, device="cuda")
+    got = solve(u)
+    del fill
+    torch.cuda.empty_cache()
+    want = solve(w)
+    assert got == want and got[0] == 0
+    torch.eq(u, w, out=eq)
+    assert bool(eq.all())
