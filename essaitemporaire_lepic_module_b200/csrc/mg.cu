@@ -585,7 +585,11 @@ __global__ void __launch_bounds__(MG_BLOCK) k_pdesolver(const MGArgs *__restrict
 // finest level, barriers and the latency of dependent FP64 operations below.
 // 512 threads: with 768 and 1024 the phases spill (128^3: 4.8 and 5.8 ms).
 constexpr int SP_BLOCK = 512;
-constexpr long long SP_SMALL = 40000;   // elements per colour one cluster solves faster than the grid
+// elements per colour up to which one cluster solves faster than the grid
+// (cold solves by the grid and by a cluster: 32x24x32, 17,000, 577 and 505 us;
+// 40x32x40, 33,100, 676 and 616; 48x40x32, 39,100, 683 and 684; 40x40x48,
+// 48,200, 705 and 713; 48^3, 67,600, 778 and 859; 56^3, 1102 and 1438)
+constexpr long long SP_SMALL = 40000;
 static_assert(MG_MAX == mgs::LEVELS, "the shared memory of their descriptors");
 
 struct SPArgs {

@@ -49,13 +49,17 @@ using Lev = mgs::Lev<float>;
 
 constexpr int XM_MAX = mgs::LEVELS;   // multigrid levels
 // threads per block: twice as many, at half the registers, on grids whose
-// finest level moves through HBM (a solve, with the cooperative groups'
-// barrier: 256^3 13.9 -> 12.7 ms, 192^3 and 176^3 the same, 160^3 10.4 -> 11.3
-// ms, 128^3 617 -> 714 us)
+// finest level moves through HBM (cold solves with electrodes, 512 and 1024
+// threads: 128^3 2.37 and 2.80 ms, 160^3 9.42 and 10.34, 192^3 6.19 and 6.32,
+// 208^3 13.10 and 12.79, 224^3 25.8 and 25.0, 256^3 11.63 and 11.17)
 constexpr int XM_BLOCK = 512, XM_BLOCK_LARGE = 1024;
-constexpr long long XM_LARGE = 3000000;   // elements per colour from which it takes those
+constexpr long long XM_LARGE = 4300000;   // elements per colour from which it takes those: between 192^3 and 208^3
 constexpr int XV = 4;           // elements per 16-byte load
-constexpr long long XM_SMALL = 60000;  // elements per colour one cluster solves faster than the grid
+// elements per colour up to which one cluster solves faster than the grid
+// (cold solves by the grid and by a cluster: 32^3, 24,500, 328 and 296 us;
+// 40x32x32, 29,400, 306 and 277; 40x32x40, 36,100, 321 and 329; 48x40x32,
+// 42,100, 356 and 380; 48x40x48, 61,400, 368 and 384; 56^3, 640 and 789)
+constexpr long long XM_SMALL = 35000;
 
 struct XArgs {
   Lev L[XM_MAX + 2];          // levels 1..ng; after them level ls + 1 with its arrays on the grid

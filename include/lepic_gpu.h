@@ -792,7 +792,7 @@ int lepic_dev_wait_selftest(long long limit_ns, void *stream);
  * given up, for tests: one cycle of lepic_dev_pdesolver with eps = 0, or
  * (mixed) one refinement of lepic_dev_pdesolver_mixed with 20,000 sweeps of the
  * coarsest level, by blocks that wait a few milliseconds at most, so that on a
- * grid solved by the whole device (above 60,000 elements per colour, 50^3)
+ * grid solved by the whole device (above 40,000 elements per colour, 42^3)
  * whose coarsest level is smoothed by one block they give up meanwhile.
  * Returns LEPIC_ERR_TIMEOUT, or without wait (mixed only) the launch status,
  * with LEPIC_ERR_TIMEOUT in the device error word; u is undefined then.  No
