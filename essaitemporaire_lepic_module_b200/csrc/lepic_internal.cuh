@@ -528,11 +528,14 @@ __device__ __forceinline__ void warp_cell_sums(int ncells, const WarpCells &S, V
 // elementary functions on the IBM RISC System/6000 processor", IBM J. Res.
 // Dev. 34, 1990: with y the rounded reciprocal and q within an ulp of a / b,
 // RN(q + RN(a - b q) y) is RN(a / b)): a y is within two ulps, one correction
-// brings it within one, the second rounds it (a zero keeps its sign, a NaN
-// stays one).  The remainders are exact for 1e-280 < |a| < 1e200 with a
-// 1e-100 < |b| < 1e100; a smaller a may end one ulp off, from a larger one
-// the result is not a number.  A branch to the division for those would cost
-// the callers' loops their registers.
+// brings it within one, the second rounds it.  The remainders are exact for
+// 1e-280 < |a| < 1e200 with a 1e-100 < |b| < 1e100; a smaller a may end one ulp
+// off, from a much larger or infinite one the result is not a number (where a
+// division has the infinity), a NaN stays one, and -0 over a positive b is +0.
+// A branch to the division for those would cost the callers' loops their
+// registers.  No caller has a use for them: positions beyond the range go
+// through quot(), a position's distance to its node is never -0, and a
+// potential that has reached 1e200 is one that diverges.
 __device__ __forceinline__ double div_by(double a, double b, double y) {
   const double q0 = a * y;
   const double q1 = __fma_rn(__fma_rn(-b, q0, a), y, q0);

@@ -1,7 +1,13 @@
 // Poisson solve of Src/pdesolver.f90 + Src/mg.f90 + Src/sors.f90 as ONE
-// persistent cooperative kernel: every V-cycle, every level, every
-// red-black sweep, the residual-ratio exit test of sor_rb and the outer
-// res/alpha < eps loop run on the device; the host sees a single launch.
+// persistent kernel: every V-cycle, every level, every red-black sweep, the
+// residual-ratio exit test of sor_rb and the outer res/alpha < eps loop run on
+// the device; the host sees a single launch.
+//
+// Two kernels with the same schedule and the same iterates, bit for bit:
+// k_pdesolver_split (the second half of this file), on colour-split copies of
+// the levels, for Dirichlet walls; k_pdesolver, the general one, on the
+// caller's arrays, for periodic and Neumann planes, for solves without
+// allocation, and where the split one does not apply (launch_split).
 //
 // Schedule (identical to the reference, one MPI rank):
 //   for each V-cycle k: down leg sor_rb(level l, dig<0) + restriction,
@@ -16,11 +22,12 @@
 // every block, so all blocks take the same exit decision and the result is
 // deterministic run to run.
 //
-// Levels with few nodes (<= SMALL_NODES) are smoothed by block 0 alone with
-// __syncthreads, avoiding grid-wide barriers on the tiny coarse grids.
+// In the general kernel levels with few nodes (<= SMALL_NODES) are smoothed by
+// block 0 alone with __syncthreads, avoiding grid-wide barriers on the tiny
+// coarse grids.
 //
 // Periodic planes in y and z (bcnd 0) and the Neumann plane at x = 0
-// (bcnd -2) run in a second instance of the kernel (GEN): the node rules of
+// (bcnd -2) run in a second instance of that kernel (GEN): the node rules of
 // Src/sors.f90:113-125, the ghost-plane refresh after each colour
 // (Src/sors.f90:157-231) and the restriction's periodic wraps
 // (Src/mg.f90:314-805); the Dirichlet instance is unchanged.
@@ -578,12 +585,16 @@ __global__ void __launch_bounds__(MG_BLOCK) k_pdesolver(const MGArgs *__restrict
 //     last smoothing of a cycle) is not computed;
 //   * the levels that fit the shared memory of one SM are smoothed there by
 //     block 0.
-// Measured (cold solves to 1e-10): 128^3 with electrodes 13.8 -> 4.4 ms (13
-// cycles; a red or black phase of level 1 takes 8 us for the 52 MB it moves
-// through L2, one of a small level 2.9 us, 1.2 of them the barrier), 40x24x32
-// 1.17 -> 0.46 ms, 96^3 warm 4.5 -> 1.0 ms.  What bounds it: L2 traffic on the
-// finest level, barriers and the latency of dependent FP64 operations below.
-// 512 threads: with 768 and 1024 the phases spill (128^3: 4.8 and 5.8 ms).
+// Measured against the general kernel: 128^3 with electrodes, cold, to 1e-10
+// 13.8 -> 4.06 ms (13 cycles; a red or black phase of level 1 takes 8 us for
+// the 52 MB it moves through L2, one of a small level 2 to 3 us with its
+// barrier); in the step loop 40x24x32 1.17 -> 0.43 ms, 96^3 4.5 -> 0.94 ms.
+// What bounds it is latency, of L2 on the finest level and of barriers and
+// dependent FP64 operations below: at 128^3 19.2 GB go through L2 at 4.8 TB/s,
+// 15 % of what it can do, the SMs issue 16 % of the time with their 16 warps
+// and the FP64 pipe is 11 % busy.
+// 512 threads: with 768 and 1024 the phases spill (128^3: 4.8 and 5.8 ms when
+// 512 took 4.4).
 constexpr int SP_BLOCK = 512;
 // elements per colour up to which one cluster solves faster than the grid
 // (cold solves by the grid and by a cluster: 32x24x32, 17,000, 577 and 505 us;

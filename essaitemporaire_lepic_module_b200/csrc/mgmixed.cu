@@ -15,9 +15,10 @@
 // All levels are colour-split (mgsplit.cuh): a red or black phase reads and
 // writes only what it needs, 16 bytes per load, and finds walls and parity in
 // one byte per element.  What bounds a solve is the number of grid phases
-// (1.2 us for the barrier alone, 2 to 3 us for a phase of a small level) and,
-// from 128^3 on, the values moved through L2.  A refinement therefore has as
-// few phases as its schedule allows:
+// (2 to 3 us for one of a small level with its barrier) and, on large grids,
+// the values moved through L2 and HBM (256^3: 41.8 GB through HBM, 0.58 of the
+// measured copy bandwidth, and 101 GB through L2).  A refinement therefore has
+// as few phases as its schedule allows:
 //   * u and b are held as colour-split FP64 copies for the solve, so the FP64
 //     residual is one phase of vector loads, which also does the first
 //     sweep's red phase (from a zero correction it needs no neighbours);
@@ -26,9 +27,9 @@
 //   * the last sweep of level 1 adds its values to u.
 // Coarse levels that fit the shared memory of one SM run there in block 0.
 // Measured against 32x8x8-node tiles staged by TMA (17 phases of about 22 us a
-// refinement at 128^3): 128^3 warm 1.53 -> 0.69 ms (4 refinements), 256^3 with
-// electrodes cold 40 -> 16.2 ms (18), 48x80x112 warm 0.72 -> 0.40 ms, 32^3
-// 0.38 -> 0.25 ms.
+// refinement at 128^3): 256^3 with electrodes cold 40 -> 11.1 ms (18
+// refinements); in the step loop 128^3 1.53 -> 0.58 ms (4), 48x80x112 0.72 ->
+// 0.34 ms, 32^3 0.38 -> 0.20 ms.
 #include <cstring>
 
 #include "mgsplit.cuh"
