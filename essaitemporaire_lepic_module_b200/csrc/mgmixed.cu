@@ -451,6 +451,36 @@ __global__ void k_wait_selftest(GridBarrier barrier, int *out_i) {
 }
 constexpr long long ROUND_NS = 900000;   // a round of looks takes 0.95 ms
 
+// A solve without device memory for the split copies (30 bytes per grid node):
+// FP64 cycles by the general kernel (12), to the same residual; the cycles
+// count as refinements.
+static int solve_without_copies(const Dims &d, const double h[3], double *u, const double *b, const int *bcnd,
+                                double eps, double omega, int ng, double eps0, int max_refine, int *iters,
+                                double *res_out, cudaStream_t s) {
+  cudaGetLastError();
+  scratch_drop("xm_");
+  if (max_refine < 1) return LEPIC_ERR_CUDA;
+  int k = 0;
+  double ktot = 0.0, res = 0.0;
+  int rc = launch_pdesolver(d, h, u, b, bcnd, max_refine, eps, omega, ng, eps0, &k, &ktot, &res, s);
+  if (rc == LEPIC_ERR_CUDA) return rc;
+  if (rc == LEPIC_OK && !(res < eps)) rc = LEPIC_ERR_NOT_CONVERGED;
+  const int hi[2] = {k - 1, rc};
+  int *out_i = (int *)scratch("xm_out_i", sizeof(int) * 4);
+  double *out_d = (double *)scratch("xm_out_d", sizeof(double) * 2);
+  if (!out_i || !out_d) return LEPIC_ERR_CUDA;
+  LEPIC_CUDA(cudaMemcpyAsync(out_i, hi, sizeof(hi), cudaMemcpyHostToDevice, s));
+  LEPIC_CUDA(cudaMemcpyAsync(out_d, &res, sizeof(double), cudaMemcpyHostToDevice, s));
+  if (!iters && !res_out) {
+    k_solve_status<<<1, 1, 0, s>>>(out_i, ctx().d_err);
+    LEPIC_CUDA(cudaGetLastError());
+    return LEPIC_OK;
+  }
+  if (iters) *iters = hi[0];
+  if (res_out) *res_out = res;
+  return rc;
+}
+
 int launch_pdesolver_mixed(const Dims &d, const double h[3], double *u, const double *b, const int *bcnd,
                            double eps, double omega, int ng, double eps0, int max_refine, int nu_fine_pre,
                            int nu_fine_post, int nu_pre, int nu_post, int coarse_sweeps, int *iters,
@@ -520,7 +550,8 @@ int launch_pdesolver_mixed(const Dims &d, const double h[3], double *u, const do
     const int halves = restricts ? 6 : 4;
     snprintf(nm, sizeof nm, "xm_%d", l);
     float *p = (float *)scratch(nm, (sizeof(float) * halves + 1) * len);
-    if (!p) return LEPIC_ERR_CUDA;
+    if (!p)
+      return solve_without_copies(d, h, u, b, bcnd, eps, omega, ng, eps0, max_refine, iters, res_out, s);
     L.red[0] = p;
     L.black = p + len;
     L.b[0] = p + 2 * len;
@@ -534,7 +565,8 @@ int launch_pdesolver_mixed(const Dims &d, const double h[3], double *u, const do
   {
     const size_t len = (size_t)A.L[1].len;
     double *p = (double *)scratch("xm_f64", sizeof(double) * 4 * len);
-    if (!p) return LEPIC_ERR_CUDA;
+    if (!p)
+      return solve_without_copies(d, h, u, b, bcnd, eps, omega, ng, eps0, max_refine, iters, res_out, s);
     for (int q = 0; q < 2; ++q) {
       A.us[q] = p + q * len;
       A.bs[q] = p + (2 + q) * len;
